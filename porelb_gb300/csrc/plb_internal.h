@@ -95,7 +95,19 @@ struct StepArgs {
     unsigned long long *err; /* min over (it << 32 | reference index) */
     unsigned int *flags;     /* bit 0: FP16 scale overflow, bit 1: fallback */
     int pf_blocks;           /* L2 prefetch distance in blocks (0 = none) */
+    int words_first;         /* load the neighbour words before waiting for the
+                                step before (see words_first_waves) */
 };
+
+/* Waves of resident CTAs up to which a step loads its words before it waits
+ * for the step before; above it, each gather goes out as its word arrives.
+ * In a short launch most CTAs start while the step before still drains, and
+ * their word loads then cost nothing (FP32: 3.3 against 3.9 us at 92k nodes,
+ * 6.8 against 7.3 at 310k; FP16 19.4 against 20.4 at 734k).  In a long one
+ * few do, and 18 words held before the first gather make the loads burstier
+ * (fixed-point FP64: 48.0 against 47.1 us at 734k nodes, 9 waves, 2% at 22M;
+ * FP32 and 16-bit: even at 30 waves, 2% slower at 115). */
+constexpr int words_first_waves(int precision) { return precision == PLB_FP64 ? 6 : 20; }
 
 /* One sample of a batch (device copy). */
 struct SampleDev {

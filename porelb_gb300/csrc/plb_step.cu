@@ -22,6 +22,7 @@
  */
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <string.h>
 
 #include "plb_emu.h"
 #include "plb_internal.h"
@@ -59,18 +60,48 @@ __device__ __forceinline__ double imul(double a, double b)
 
 /* ------------------------------------------------------------- gather */
 
-template <typename T>
-__device__ __forceinline__ T ldg_t(const T *p) { return __ldg(p); }
+/* A step's launch overlaps the one before it (programmatic dependent
+ * launch): its CTAs start while the last wave of the previous step drains,
+ * read what no step writes (the neighbour words, the block maps) and then
+ * wait for the previous grid to complete and its stores to be visible.  So
+ * nothing before pdl_wait() may read distributions or write anything, and
+ * the distributions, which the previous grid may still be writing when this
+ * one starts, are read with plain loads, not through the read-only path. */
+__device__ __forceinline__ void pdl_launch_next()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
+__device__ __forceinline__ void load_words(const uint32_t *nbr, long long np, long long i,
+                                           int (&w)[Q - 1])
+{
+#pragma unroll
+    for (int j = 0; j < Q - 1; j++) w[j] = (int)__ldg(nbr + (long long)j * np + i);
+}
+
+template <typename T>
+__device__ __forceinline__ void gather_words(const T *fin, long long np, long long i,
+                                             const int (&w)[Q - 1], T (&f)[Q])
+{
+    f[0] = fin[i];
+#pragma unroll
+    for (int j = 1; j < Q; j++) f[j] = fin[(long long)j * np + w[j - 1]];
+}
+
+/* the same two in one: each gather goes out as its word arrives */
 template <typename T>
 __device__ __forceinline__ void gather(const T *fin, const uint32_t *nbr,
                                        long long np, long long i, T (&f)[Q])
 {
-    f[0] = ldg_t(fin + i);
+    f[0] = fin[i];
 #pragma unroll
     for (int j = 1; j < Q; j++) {
         const int w = (int)__ldg(nbr + (long long)(j - 1) * np + i);
-        f[j] = ldg_t(fin + ((long long)j * np + w));
+        f[j] = fin[(long long)j * np + w];
     }
 }
 
@@ -443,21 +474,6 @@ __device__ __forceinline__ Macro collide_node(T (&raw)[Q], const T *fin, T *fout
     return m;
 }
 
-/* Gather, collide and store node i.  Returns the macros; dev_max receives
- * the largest stored deviation magnitude of the 16-bit forms. */
-template <int PREC, bool MACRO>
-__device__ __forceinline__ Macro step_node(const void *fin_, void *fout_,
-                                           const uint32_t *nbr, long long np,
-                                           long long i, const Coeffs &co,
-                                           unsigned int &flags, float &dev_max)
-{
-    using T = typename StoreOf<PREC>::T;
-    const T *fin = (const T *)fin_;
-    T raw[Q];
-    gather<T>(fin, nbr, np, i, raw);
-    return collide_node<PREC, MACRO>(raw, fin, (T *)fout_, nbr, np, i, co, flags, dev_max);
-}
-
 /* Bulk L2 prefetch of [p, p + bytes), bytes a positive multiple of 16 and
  * p 16-byte aligned. */
 __device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes)
@@ -498,12 +514,24 @@ k_step(const StepArgs a)
                                                   a.nbr, a.npad, a.n,
                                                   (long long)blockIdx.x + a.pf_blocks,
                                                   blockDim.x);
+    using T = typename StoreOf<PREC>::T;
+    T raw[Q];
+    pdl_launch_next();
+    if (a.words_first) {
+        int w[Q - 1];
+        if (i < a.n) load_words(a.nbr, a.npad, i, w);
+        pdl_wait();
+        if (i < a.n) gather_words<T>((const T *)a.fin, a.npad, i, w, raw);
+    } else {
+        pdl_wait();
+        if (i < a.n) gather<T>((const T *)a.fin, a.nbr, a.npad, i, raw);
+    }
     double sum_u = 0.0, sum_r = 0.0;
     if (i < a.n) {
         float dm = 0.f;
         unsigned int fl = 0;
-        const Macro m = step_node<PREC, MACRO>(a.fin, a.fout, a.nbr, a.npad, i, a.co,
-                                               fl, dm);
+        const Macro m = collide_node<PREC, MACRO>(raw, (const T *)a.fin, (T *)a.fout, a.nbr,
+                                                  a.npad, i, a.co, fl, dm);
         if (fl) atomicOr(a.flags, fl);
         if (m.bad) {
             const unsigned long long key =
@@ -633,6 +661,24 @@ k_batch_step(const BatchArgs a)
     }
 }
 
+/* One step launch, overlapping the kernel before it in the stream (see
+ * pdl_wait). */
+static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, const StepArgs &a,
+                              cudaStream_t s)
+{
+    cudaLaunchConfig_t c;
+    memset(&c, 0, sizeof(c));
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, fn, a);
+}
+
 template <int PREC>
 static cudaError_t launch_prec(bool macros, const StepArgs &a, int block,
                                int variant, cudaStream_t s)
@@ -644,19 +690,15 @@ static cudaError_t launch_prec(bool macros, const StepArgs &a, int block,
                            PREC == PLB_BF16DEV;
     if constexpr (tuned) {
         if (variant == 1) {
-            if (macros) k_step<PREC, true, 1><<<grid, block, 0, s>>>(a);
-            else k_step<PREC, false, 1><<<grid, block, 0, s>>>(a);
-            return cudaGetLastError();
+            return launch_pdl(macros ? k_step<PREC, true, 1> : k_step<PREC, false, 1>, grid,
+                              block, a, s);
         }
         if (variant == 3) {
-            if (macros) k_step<PREC, true, 3><<<grid, block, 0, s>>>(a);
-            else k_step<PREC, false, 3><<<grid, block, 0, s>>>(a);
-            return cudaGetLastError();
+            return launch_pdl(macros ? k_step<PREC, true, 3> : k_step<PREC, false, 3>, grid,
+                              block, a, s);
         }
     }
-    if (macros) k_step<PREC, true, 0><<<grid, block, 0, s>>>(a);
-    else k_step<PREC, false, 0><<<grid, block, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(macros ? k_step<PREC, true, 0> : k_step<PREC, false, 0>, grid, block, a, s);
 }
 
 /* Blocks of the (non-macro) step kernel resident on the whole device at

@@ -1,0 +1,33 @@
+"""Steps of one call overlap each other on the device (a step's CTAs start
+while the step before drains).  One call of many steps and the same steps
+one call at a time, each waited for, have to give the same bits: at the
+sizes where the default CTA changes (one CTA per SM still covers the domain
+with half the threads) and on both sides of the number of waves up to which
+the neighbour words are loaded before the wait."""
+import numpy as np
+import pytest
+
+import porelb_gb300 as P
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision,dims", [
+    ("fp64_exact", (9, 8, 7)), ("fp64_exact", (24, 31, 33)), ("fp64_exact", (37, 36, 41)),
+    ("fp64_exact", (161, 160, 162)), ("fp64_exact", (166, 165, 167)),
+    ("fp64", (30, 31, 31)), ("fp64", (108, 110, 111)), ("fp64", (112, 113, 114)),
+    ("fp64_fma", (31, 30, 30)), ("fp32", (29, 31, 30)), ("fp32", (222, 221, 222)),
+    ("fp32", (226, 225, 226)), ("fp16dev", (40, 41, 39)), ("bf16dev", (228, 226, 227))])
+def test_one_call_equals_waited_steps(precision, dims):
+    steps = 7
+    out = []
+    for chunks in ([steps], [1] * steps):
+        with P.Simulation.packed(5, *dims, 0.3 + min(dims) / 40, 1.0 + min(dims) / 20, 0.35,
+                                 tau=0.7, force=1e-5, precision=precision) as sim:
+            sim.init_dist_macro()
+            for c in chunks:
+                sim.step(c)
+            out.append((sim.N, sim.macros().copy(), sim.permeability()))
+    assert out[0][0] == out[1][0] > 0
+    assert np.array_equal(out[0][1], out[1][1])
+    assert out[0][2] == out[1][2]
