@@ -662,8 +662,8 @@ static cudaError_t step_chain(plb_batch *b, bool grouped, int grid,
         a.grp_cur = b->gcur;
     }
     const int bt = b->cta;
-    const void *fn = batch_step_kernel(b->precision, false, bt);
-    const void *fn_m = batch_step_kernel(b->precision, true, bt);
+    const void *fn = batch_step_kernel(b->precision, false, bt, grid);
+    const void *fn_m = batch_step_kernel(b->precision, true, bt, grid);
     args.assign((size_t)b->K, a);
     nodes.assign((size_t)b->K, nullptr);
     cudaGraph_t g = nullptr;
@@ -683,8 +683,14 @@ static cudaError_t step_chain(plb_batch *b, bool grouped, int grid,
         p.gridDim = dim3((unsigned)(grid > 0 ? grid : 1));
         p.blockDim = dim3((unsigned)bt);
         p.kernelParams = kp;
-        e = cudaGraphAddKernelNode(&nodes[(size_t)k], g, prev ? &prev : nullptr,
-                                   prev ? 1 : 0, &p);
+        e = cudaGraphAddKernelNode(&nodes[(size_t)k], g, nullptr, 0, &p);
+        /* each step starts while the one before drains (pdl_wait) */
+        cudaGraphEdgeData over;
+        memset(&over, 0, sizeof(over));
+        over.from_port = cudaGraphKernelNodePortProgrammatic;
+        over.type = cudaGraphDependencyTypeProgrammatic;
+        if (e == cudaSuccess && prev)
+            e = cudaGraphAddDependencies(g, &prev, &nodes[(size_t)k], &over, 1);
         prev = nodes[(size_t)k];
     }
     if (grouped && e == cudaSuccess) {
@@ -790,8 +796,8 @@ static int set_chain_grid(plb_batch *b, cudaGraphExec_t exec, std::vector<BatchA
                           std::vector<cudaGraphNode_t> &nodes, int grid)
 {
     const int bt = b->cta;
-    const void *fn = batch_step_kernel(b->precision, false, bt);
-    const void *fn_m = batch_step_kernel(b->precision, true, bt);
+    const void *fn = batch_step_kernel(b->precision, false, bt, grid);
+    const void *fn_m = batch_step_kernel(b->precision, true, bt, grid);
     for (int k = 0; k < b->K; k++) {
         void *kp[1] = {&args[(size_t)k]};
         cudaKernelNodeParams p;

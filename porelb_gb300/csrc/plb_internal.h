@@ -169,9 +169,10 @@ cudaError_t launch_step(int precision, bool macros, const StepArgs &a,
 
 /* The batch step kernel (one BatchArgs argument) of a storage form with
  * CTAs of `cta` threads (128 or 256; pool blocks of 256 nodes, 256 / cta
- * CTAs each), for a graph kernel node; NULL for another size. */
+ * CTAs each) for a launch of `grid` CTAs, for a graph kernel node; NULL for
+ * another size. */
 constexpr int kBatchBlock = 256;
-const void *batch_step_kernel(int precision, bool macros, int cta);
+const void *batch_step_kernel(int precision, bool macros, int cta, int grid);
 
 /* Fill the coefficients from tau, F and the storage scale. */
 void make_coeffs(double tau, double force, float scale, Coeffs *c);

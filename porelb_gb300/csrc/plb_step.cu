@@ -105,6 +105,24 @@ __device__ __forceinline__ void gather(const T *fin, const uint32_t *nbr,
     }
 }
 
+/* The streamed values of node i (if valid), after the step before: WF loads
+ * the neighbour words before the wait, else each gather goes out as its word
+ * arrives after it (words_first_waves). */
+template <typename T, bool WF>
+__device__ __forceinline__ void stream_node(const void *fin, const uint32_t *nbr,
+                                            long long np, long long i, bool valid, T (&f)[Q])
+{
+    if constexpr (WF) {
+        int w[Q - 1];
+        if (valid) load_words(nbr, np, i, w);
+        pdl_wait();
+        if (valid) gather_words<T>((const T *)fin, np, i, w, f);
+    } else {
+        pdl_wait();
+        if (valid) gather<T>((const T *)fin, nbr, np, i, f);
+    }
+}
+
 /* ------------------------------------------------- FP64, reference order */
 
 /* e.u as the reference evaluates ((e0*u + e1*v) + e2*w) (porelb.c:9): terms
@@ -504,7 +522,7 @@ __device__ __forceinline__ void prefetch_block(const T *fin, const uint32_t *nbr
     for (int j = 0; j < Q; j++) prefetch_l2(fin + (long long)j * np + i0, fb);
 }
 
-template <int PREC, bool MACRO, int VARIANT>
+template <int PREC, bool MACRO, int VARIANT, bool WF>
 __global__ void __launch_bounds__(256, MinBlocks<PREC, VARIANT>::v)
 k_step(const StepArgs a)
 {
@@ -517,14 +535,15 @@ k_step(const StepArgs a)
     using T = typename StoreOf<PREC>::T;
     T raw[Q];
     pdl_launch_next();
-    if (a.words_first) {
-        int w[Q - 1];
-        if (i < a.n) load_words(a.nbr, a.npad, i, w);
-        pdl_wait();
-        if (i < a.n) gather_words<T>((const T *)a.fin, a.npad, i, w, raw);
+    if constexpr (PREC == PLB_FP64) {
+        /* one kernel for both: built apart, the form with the words after
+         * the wait spills 20 B at its 128 registers (348 against 341 us at
+         * 256^3); FP32 and 16-bit kernels are the ones with registers to
+         * lose to a branch */
+        if (a.words_first) stream_node<T, true>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
+        else stream_node<T, false>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
     } else {
-        pdl_wait();
-        if (i < a.n) gather<T>((const T *)a.fin, a.nbr, a.npad, i, raw);
+        stream_node<T, WF>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
     }
     double sum_u = 0.0, sum_r = 0.0;
     if (i < a.n) {
@@ -574,7 +593,7 @@ k_step(const StepArgs a)
  * that run at the same time work on neighbouring pool blocks, so in Morton
  * order their gathers share L2 lines (a fixed grid looping over the list
  * lost that and ran 23% slower in the FP64 form). */
-template <int PREC, bool MACRO, int BT>
+template <int PREC, bool MACRO, int BT, bool WF>
 __global__ void __launch_bounds__(BT, MinBlocks<PREC, 0>::v * (kBatchBlock / BT))
 k_batch_step(const BatchArgs a)
 {
@@ -604,9 +623,12 @@ k_batch_step(const BatchArgs a)
     }
     double sum_u = 0.0, sum_r = 0.0;
     float dmax = 0.f;
-    /* the gathers first: they need only the node's place in the pool */
+    /* the gathers first: they need only the node's place in the pool.  The
+     * block maps and words above and below are the interval's: no step
+     * writes them, so they are read before the wait (see k_step) */
     T raw[Q];
-    if (valid) gather<T>((const T *)a.fin, a.nbr, a.npad, i, raw);
+    pdl_launch_next();
+    stream_node<T, WF>(a.fin, a.nbr, a.npad, i, valid, raw);
     if (valid) {
         {
             /* the sample's coefficients straight from global memory (the
@@ -679,26 +701,33 @@ static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, const S
     return cudaLaunchKernelEx(&c, fn, a);
 }
 
+template <int PREC, int V>
+static void (*step_fn(bool macros, bool wf))(StepArgs)
+{
+    if constexpr (PREC != PLB_FP64)
+        if (wf) return macros ? k_step<PREC, true, V, true> : k_step<PREC, false, V, true>;
+    return macros ? k_step<PREC, true, V, false> : k_step<PREC, false, V, false>;
+}
+
+/* the tighter register budgets are built for the tuned forms only */
+template <int PREC>
+static void (*step_variant(bool macros, bool wf, int variant))(StepArgs)
+{
+    if constexpr (PREC == PLB_FP64 || PREC == PLB_FP32 || PREC == PLB_FP16DEV ||
+                  PREC == PLB_BF16DEV) {
+        if (variant == 1) return step_fn<PREC, 1>(macros, wf);
+        if (variant == 3) return step_fn<PREC, 3>(macros, wf);
+    }
+    return step_fn<PREC, 0>(macros, wf);
+}
+
 template <int PREC>
 static cudaError_t launch_prec(bool macros, const StepArgs &a, int block,
                                int variant, cudaStream_t s)
 {
     const int grid = (a.n + block - 1) / block;
     if (grid == 0) return cudaSuccess;
-    /* the tighter budgets are built for the tuned forms only */
-    constexpr bool tuned = PREC == PLB_FP64 || PREC == PLB_FP32 || PREC == PLB_FP16DEV ||
-                           PREC == PLB_BF16DEV;
-    if constexpr (tuned) {
-        if (variant == 1) {
-            return launch_pdl(macros ? k_step<PREC, true, 1> : k_step<PREC, false, 1>, grid,
-                              block, a, s);
-        }
-        if (variant == 3) {
-            return launch_pdl(macros ? k_step<PREC, true, 3> : k_step<PREC, false, 3>, grid,
-                              block, a, s);
-        }
-    }
-    return launch_pdl(macros ? k_step<PREC, true, 0> : k_step<PREC, false, 0>, grid, block, a, s);
+    return launch_pdl(step_variant<PREC>(macros, a.words_first != 0, variant), grid, block, a, s);
 }
 
 /* Blocks of the (non-macro) step kernel resident on the whole device at
@@ -706,13 +735,7 @@ static cudaError_t launch_prec(bool macros, const StepArgs &a, int block,
 template <int PREC>
 static int wave_prec(int block, int variant)
 {
-    const void *fn = (const void *)k_step<PREC, false, 0>;
-    constexpr bool tuned = PREC == PLB_FP64 || PREC == PLB_FP32 || PREC == PLB_FP16DEV ||
-                           PREC == PLB_BF16DEV;
-    if constexpr (tuned) {
-        if (variant == 1) fn = (const void *)k_step<PREC, false, 1>;
-        if (variant == 3) fn = (const void *)k_step<PREC, false, 3>;
-    }
+    const void *fn = (const void *)step_variant<PREC>(false, false, variant);
     int dev = 0, sms = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -748,7 +771,7 @@ static int batch_wave_bt()
     int dev = 0, sms = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<PREC, false, BT>, BT,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<PREC, false, BT, true>, BT,
                                                       0) != cudaSuccess)
         return 0;
     return sms * per;
@@ -773,26 +796,39 @@ int batch_wave_blocks(int precision, int cta)
     }
 }
 
-template <int PREC>
-static const void *batch_fn(bool macros, int cta)
+template <int PREC, int BT>
+static const void *batch_fn(bool macros, bool wf)
 {
-    if (cta == 128)
-        return macros ? (const void *)k_batch_step<PREC, true, 128>
-                      : (const void *)k_batch_step<PREC, false, 128>;
-    return macros ? (const void *)k_batch_step<PREC, true, kBatchBlock>
-                  : (const void *)k_batch_step<PREC, false, kBatchBlock>;
+    if constexpr (PREC == PLB_FP16DEV || PREC == PLB_BF16DEV) {
+        if (!wf)
+            return macros ? (const void *)k_batch_step<PREC, true, BT, false>
+                          : (const void *)k_batch_step<PREC, false, BT, false>;
+    }
+    return macros ? (const void *)k_batch_step<PREC, true, BT, true>
+                  : (const void *)k_batch_step<PREC, false, BT, true>;
 }
 
-const void *batch_step_kernel(int precision, bool macros, int cta)
+/* The pool's words come first in every launch of the forms of 4 and 8 bytes
+ * (pools of 0.1M to 6M nodes: FP64 3-6% faster than words after the wait,
+ * FP32 even to 10%); the 16-bit forms', up to the same number of waves as a
+ * plain step's (0.1M nodes 3.2 against 3.6 us, 5M nodes 132 against 130). */
+template <int PREC>
+static const void *batch_fn_cta(bool macros, int cta, int grid)
+{
+    const bool wf = grid <= (long long)words_first_waves(PREC) * batch_wave_prec<PREC>(cta);
+    return cta == 128 ? batch_fn<PREC, 128>(macros, wf) : batch_fn<PREC, kBatchBlock>(macros, wf);
+}
+
+const void *batch_step_kernel(int precision, bool macros, int cta, int grid)
 {
     if (cta != 128 && cta != kBatchBlock) return nullptr;
     switch (precision) {
-    case PLB_FP64_EXACT: return batch_fn<PLB_FP64_EXACT>(macros, cta);
-    case PLB_FP64: return batch_fn<PLB_FP64>(macros, cta);
-    case PLB_FP64_FMA: return batch_fn<PLB_FP64_FMA>(macros, cta);
-    case PLB_FP32: return batch_fn<PLB_FP32>(macros, cta);
-    case PLB_FP16DEV: return batch_fn<PLB_FP16DEV>(macros, cta);
-    case PLB_BF16DEV: return batch_fn<PLB_BF16DEV>(macros, cta);
+    case PLB_FP64_EXACT: return batch_fn_cta<PLB_FP64_EXACT>(macros, cta, grid);
+    case PLB_FP64: return batch_fn_cta<PLB_FP64>(macros, cta, grid);
+    case PLB_FP64_FMA: return batch_fn_cta<PLB_FP64_FMA>(macros, cta, grid);
+    case PLB_FP32: return batch_fn_cta<PLB_FP32>(macros, cta, grid);
+    case PLB_FP16DEV: return batch_fn_cta<PLB_FP16DEV>(macros, cta, grid);
+    case PLB_BF16DEV: return batch_fn_cta<PLB_BF16DEV>(macros, cta, grid);
     default: return nullptr;
     }
 }

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import porelb_gb300 as P
+from porelb_gb300.batch import Batch
 
 pytestmark = pytest.mark.gpu
 
@@ -31,3 +32,22 @@ def test_one_call_equals_waited_steps(precision, dims):
     assert out[0][0] == out[1][0] > 0
     assert np.array_equal(out[0][1], out[1][1])
     assert out[0][2] == out[1][2]
+
+
+@pytest.mark.parametrize("precision,edge", [("fp16dev", 226), ("bf16dev", 226), ("fp32", 64),
+                                            ("fp64", 110)])
+def test_sample_alone_equals_sample_in_a_long_launch(precision, edge):
+    """Pool launches of few and of many waves take different kernels in the
+    16-bit forms: a small sample's bits are the same in both."""
+    out = []
+    for mates in (0, 1):
+        with Batch(int(mates * edge ** 3 * 0.36) + 40000, 2, precision, check_every=20) as pool:
+            sid = pool.add_packed(3, 33, 31, 32, 3.0, 5.0, 0.4, 0.9, 1e-6, tol=0.0,
+                                  max_steps=1000)
+            for _ in range(mates):
+                pool.add_packed(4, edge, edge, edge, 5.0, 10.0, 0.35, 0.8, 1e-6, tol=0.0,
+                                max_steps=1000)
+            pool.run(2)
+            out.append((pool.get_f(sid), pool.result(sid)))
+    assert np.array_equal(out[0][0], out[1][0])
+    assert out[0][1] == out[1][1]
