@@ -157,15 +157,27 @@ int flag_tables(const uint8_t *dflag, int nx, int ny, int nz, int num_p,
                 uint16_t *coord, uint32_t *nbr, uint32_t word_base,
                 uint32_t rest_word, cudaStream_t st);
 
-/* Launch one step of the given precision. */
-/* blocks of the step kernel resident on the device at once (0 if unknown) */
-int step_wave_blocks(int precision, int block, int variant);
-/* the same for the batch step kernel with CTAs of `cta` threads */
+/* Launch shape of a handle's steps. */
+struct StepLaunch {
+    int block;       /* threads per CTA */
+    int variant;     /* register budget (plb_params.kernel_variant) */
+    int wave;        /* CTAs resident on the device at once (0: not planned) */
+    int words_first; /* as StepArgs */
+    int smem;        /* shared memory that spreads the grid over the SMs */
+};
+
+/* default threads per CTA of the step on n nodes (current device) */
+int step_block(int precision, int n);
+/* fill in the rest of the shape for n nodes, given block and variant */
+void plan_step(int precision, int n, StepLaunch *l);
+/* launch one step of the given precision */
+cudaError_t launch_step(int precision, bool macros, const StepArgs &a, const StepLaunch &l,
+                        cudaStream_t s);
+/* CTAs of `cta` threads of the batch step kernel resident on the device at
+ * once (0 if unknown) */
 int batch_wave_blocks(int precision, int cta);
 /* default threads per CTA of the batch step (128 or 256) */
 int batch_default_cta(int precision);
-cudaError_t launch_step(int precision, bool macros, const StepArgs &a,
-                        int block, int variant, cudaStream_t s);
 
 /* The batch step kernel (one BatchArgs argument) of a storage form with
  * CTAs of `cta` threads (128 or 256; pool blocks of 256 nodes, 256 / cta
@@ -173,6 +185,8 @@ cudaError_t launch_step(int precision, bool macros, const StepArgs &a,
  * another size. */
 constexpr int kBatchBlock = 256;
 const void *batch_step_kernel(int precision, bool macros, int cta, int grid);
+/* its shared memory (see spread_smem) */
+int batch_step_smem(int precision, int cta, int grid);
 
 /* Fill the coefficients from tau, F and the storage scale. */
 void make_coeffs(double tau, double force, float scale, Coeffs *c);

@@ -30,7 +30,8 @@ struct plb_sim {
     int n, nx, ny, nz, num_p;
     long long npad;
     int precision, ordering, halo, block, boundary, variant;
-    int prefetch, wave; /* L2 prefetch on; resident blocks (0 = not queried) */
+    int prefetch;     /* L2 prefetch on */
+    StepLaunch shape; /* launch shape (planned at the first step) */
     int device;
     cudaStream_t stream;
     void *f[2];
@@ -706,22 +707,6 @@ done:
     return rc;
 }
 
-/* Threads per CTA of the step: 128 for the fixed-point FP64 form, 256
- * otherwise (4% apart at 256^3), halved down to 64 while one CTA per SM
- * still covers the domain: fewer warps then share an SM's pipes, and the
- * step is one CTA's latency (1.4k-4.8k nodes, 256 -> 64 threads: bit-exact
- * form 21.1 -> 15.0 us, FMA form 13.5 -> 7.1, FP32 2.08 -> 1.77; at 38.7k
- * nodes, one 256-thread CTA per SM, halving again loses: 21.2 against 25.2 us,
- * FP32 2.39 against 2.64). */
-static int default_block(int precision, int n, int device)
-{
-    int block = precision == PLB_FP64 ? 128 : 256, sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-        sms = 0;
-    while (block > 64 && n <= (long long)sms * (block / 2)) block /= 2;
-    return block;
-}
-
 /* Validate the parameters, create the handle and allocate its device arrays
  * for n nodes (everything but the tables). */
 static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
@@ -764,7 +749,7 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
      * GB300 - every tighter budget spills: 96 to 120 registers ran at 13.5 to
      * 15.2 GLUPS at 256^3 against 16.2) */
     s->variant = p->kernel_variant == 1 ? 1 : (p->kernel_variant == 3 ? 3 : 0);
-    s->block = p->block_size > 0 ? p->block_size : default_block(p->precision, n, p->device);
+    s->block = p->block_size > 0 ? p->block_size : step_block(p->precision, n);
     if (s->block > 256 || (s->block & 31)) s->block = 256;
     /* prefetching the next wave into L2 pays for the issue-bound FP64 form
      * (+5% at 256^3 and 512^3) and costs the bandwidth-bound forms (FP32
@@ -1021,17 +1006,21 @@ int plb_step_async(plb_sim *s, int it_begin, int nsteps)
     a.partial = s->partial;
     a.err = s->err;
     a.flags = s->flags;
-    if (s->wave == 0) s->wave = step_wave_blocks(s->precision, s->block, s->variant);
+    if (s->shape.wave == 0) {
+        s->shape.block = s->block;
+        s->shape.variant = s->variant;
+        plan_step(s->precision, s->n, &s->shape);
+    }
+    a.words_first = s->shape.words_first;
     /* half a wave of resident blocks ahead (measured at 256^3 and 512^3:
      * +0.7% against a whole wave, +7% against no prefetch) */
-    a.pf_blocks = s->prefetch ? (s->wave + 1) / 2 : 0;
-    a.words_first = s->nblocks <= words_first_waves(s->precision) * (long long)s->wave;
+    a.pf_blocks = s->prefetch ? (s->shape.wave + 1) / 2 : 0;
     for (int k = 0; k < nsteps; k++) {
         a.fin = s->f[s->cur];
         a.fout = s->f[s->cur ^ 1];
         a.co.it = it_begin + k;
         const bool last = (k == nsteps - 1);
-        cudaError_t e = launch_step(s->precision, last, a, s->block, s->variant, s->stream);
+        cudaError_t e = launch_step(s->precision, last, a, s->shape, s->stream);
         if (e != cudaSuccess) {
             fprintf(stderr, "porelb_gpu: step launch failed: %s\n", cudaGetErrorString(e));
             return PLB_ERR_CUDA;

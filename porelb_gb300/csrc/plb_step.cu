@@ -685,13 +685,14 @@ k_batch_step(const BatchArgs a)
 
 /* One step launch, overlapping the kernel before it in the stream (see
  * pdl_wait). */
-static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, const StepArgs &a,
-                              cudaStream_t s)
+static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, int smem,
+                              const StepArgs &a, cudaStream_t s)
 {
     cudaLaunchConfig_t c;
     memset(&c, 0, sizeof(c));
     c.gridDim = dim3((unsigned)grid);
     c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = (size_t)smem;
     c.stream = s;
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -699,6 +700,47 @@ static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, const S
     c.attrs = &at;
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, fn, a);
+}
+
+/* Shared memory a step CTA asks for (and does not use) so that an SM holds
+ * no more CTAs than an even spread of the grid gives it.  While a step's
+ * CTAs start among the last of the step before, the free SMs take several
+ * each and the rest none: at 16k to 76k nodes a step then took up to twice
+ * its time (at 16k nodes FP64 5.4 against 3.0 us, FMA form 27 / 7.7; FP32 at
+ * 76k 4.1 / 2.8).  The requests only cap the residency; a grid that needs every CTA slot of an SM keeps all of its L1
+ * (FP32 at 179k nodes: 4.3 us, capped 4.8).  0 = no cap. */
+template <typename Fn>
+static int spread_smem(Fn fn, Fn fn_macros, int grid, int block)
+{
+    int dev = 0, sms = 0, per = 0, total = 0, reserved = 0, most = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)fn, block, 0) !=
+            cudaSuccess ||
+        sms <= 0 || grid <= 0)
+        return 0;
+    const int share = (grid + sms - 1) / sms;
+    if (share >= per) return 0;
+    /* the macro kernels' own static shared memory (under 1 KB) comes on top */
+    const int slack = 1024;
+    int smem = (total / share - reserved - slack) / 1024 * 1024;
+    if (smem > most - slack) smem = most - slack;
+    /* the same limit whatever the grid: handles of other sizes and threads
+     * set it too */
+    if (cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - slack) != cudaSuccess ||
+        cudaFuncSetAttribute((const void *)fn_macros, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - slack) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return smem;
 }
 
 template <int PREC, int V>
@@ -722,38 +764,79 @@ static void (*step_variant(bool macros, bool wf, int variant))(StepArgs)
 }
 
 template <int PREC>
-static cudaError_t launch_prec(bool macros, const StepArgs &a, int block,
-                               int variant, cudaStream_t s)
+static cudaError_t launch_prec(bool macros, const StepArgs &a, const StepLaunch &l,
+                               cudaStream_t s)
 {
-    const int grid = (a.n + block - 1) / block;
+    const int grid = (a.n + l.block - 1) / l.block;
     if (grid == 0) return cudaSuccess;
-    return launch_pdl(step_variant<PREC>(macros, a.words_first != 0, variant), grid, block, a, s);
+    return launch_pdl(step_variant<PREC>(macros, a.words_first != 0, l.variant), grid, l.block,
+                      l.smem, a, s);
 }
 
-/* Blocks of the (non-macro) step kernel resident on the whole device at
- * once: the L2 prefetch distance. */
-template <int PREC>
-static int wave_prec(int block, int variant)
+/* CTAs of a kernel resident on an SM of the current device, and its SMs;
+ * false if unknown. */
+static bool occupancy(const void *fn, int block, int *per, int *sms)
 {
-    const void *fn = (const void *)step_variant<PREC>(false, false, variant);
-    int dev = 0, sms = 0, per = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, block, 0) != cudaSuccess)
-        return 0;
-    return sms * per;
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, fn, block, 0) == cudaSuccess;
 }
 
-int step_wave_blocks(int precision, int block, int variant)
+template <int PREC>
+static void plan_prec(int n, StepLaunch *l)
+{
+    int per = 0, sms = 0;
+    const int grid = (n + l->block - 1) / l->block;
+    /* blocks of the (non-macro) kernel resident on the whole device at once:
+     * the L2 prefetch distance */
+    l->wave = occupancy((const void *)step_variant<PREC>(false, false, l->variant), l->block,
+                        &per, &sms) ? sms * per : 0;
+    l->words_first = grid <= words_first_waves(PREC) * (long long)l->wave;
+    l->smem = spread_smem(step_variant<PREC>(false, l->words_first != 0, l->variant),
+                          step_variant<PREC>(true, l->words_first != 0, l->variant), grid,
+                          l->block);
+}
+
+void plan_step(int precision, int n, StepLaunch *l)
 {
     switch (precision) {
-    case PLB_FP64_EXACT: return wave_prec<PLB_FP64_EXACT>(block, variant);
-    case PLB_FP64: return wave_prec<PLB_FP64>(block, variant);
-    case PLB_FP64_FMA: return wave_prec<PLB_FP64_FMA>(block, variant);
-    case PLB_FP32: return wave_prec<PLB_FP32>(block, variant);
-    case PLB_FP16DEV: return wave_prec<PLB_FP16DEV>(block, variant);
-    case PLB_BF16DEV: return wave_prec<PLB_BF16DEV>(block, variant);
-    default: return 0;
+    case PLB_FP64_EXACT: return plan_prec<PLB_FP64_EXACT>(n, l);
+    case PLB_FP64: return plan_prec<PLB_FP64>(n, l);
+    case PLB_FP64_FMA: return plan_prec<PLB_FP64_FMA>(n, l);
+    case PLB_FP32: return plan_prec<PLB_FP32>(n, l);
+    case PLB_FP16DEV: return plan_prec<PLB_FP16DEV>(n, l);
+    case PLB_BF16DEV: return plan_prec<PLB_BF16DEV>(n, l);
+    default: return;
+    }
+}
+
+/* Threads per CTA of the plain step.  128 for the fixed-point and FMA FP64
+ * forms; 256 for the others once 128-thread CTAs fill the device (FP16 at
+ * 22M nodes 575 against 648 us), and 128 below, where the finer grain
+ * spreads better (FP32 at 131k nodes 3.8 against 4.2 us).  Domains that 64-thread CTAs cover with one
+ * per SM take those: fewer warps share an SM's pipes (1.4k-9k nodes: FMA 7.0
+ * against 7.7 us, FP64 2.8 / 3.1). */
+template <int PREC>
+static int block_prec(int n)
+{
+    int per = 0, sms = 0;
+    if (!occupancy((const void *)step_variant<PREC>(false, false, 0), 128, &per, &sms)) return 256;
+    if (n <= sms * 64) return 64;
+    if (PREC == PLB_FP64 || PREC == PLB_FP64_FMA) return 128;
+    return n <= (long long)sms * per * 128 ? 128 : 256;
+}
+
+int step_block(int precision, int n)
+{
+    switch (precision) {
+    case PLB_FP64_EXACT: return block_prec<PLB_FP64_EXACT>(n);
+    case PLB_FP64: return block_prec<PLB_FP64>(n);
+    case PLB_FP64_FMA: return block_prec<PLB_FP64_FMA>(n);
+    case PLB_FP32: return block_prec<PLB_FP32>(n);
+    case PLB_FP16DEV: return block_prec<PLB_FP16DEV>(n);
+    case PLB_BF16DEV: return block_prec<PLB_BF16DEV>(n);
+    default: return 256;
     }
 }
 
@@ -768,13 +851,9 @@ int batch_default_cta(int precision)
 template <int PREC, int BT>
 static int batch_wave_bt()
 {
-    int dev = 0, sms = 0, per = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<PREC, false, BT, true>, BT,
-                                                      0) != cudaSuccess)
-        return 0;
-    return sms * per;
+    int per = 0, sms = 0;
+    return occupancy((const void *)k_batch_step<PREC, false, BT, true>, BT, &per, &sms) ? sms * per
+                                                                                      : 0;
 }
 
 template <int PREC>
@@ -819,6 +898,13 @@ static const void *batch_fn_cta(bool macros, int cta, int grid)
     return cta == 128 ? batch_fn<PREC, 128>(macros, wf) : batch_fn<PREC, kBatchBlock>(macros, wf);
 }
 
+int batch_step_smem(int precision, int cta, int grid)
+{
+    const void *fn = batch_step_kernel(precision, false, cta, grid);
+    const void *fn_m = batch_step_kernel(precision, true, cta, grid);
+    return fn && fn_m ? spread_smem(fn, fn_m, grid, cta) : 0;
+}
+
 const void *batch_step_kernel(int precision, bool macros, int cta, int grid)
 {
     if (cta != 128 && cta != kBatchBlock) return nullptr;
@@ -833,16 +919,16 @@ const void *batch_step_kernel(int precision, bool macros, int cta, int grid)
     }
 }
 
-cudaError_t launch_step(int precision, bool macros, const StepArgs &a,
-                        int block, int variant, cudaStream_t s)
+cudaError_t launch_step(int precision, bool macros, const StepArgs &a, const StepLaunch &l,
+                        cudaStream_t s)
 {
     switch (precision) {
-    case PLB_FP64_EXACT: return launch_prec<PLB_FP64_EXACT>(macros, a, block, variant, s);
-    case PLB_FP64: return launch_prec<PLB_FP64>(macros, a, block, variant, s);
-    case PLB_FP64_FMA: return launch_prec<PLB_FP64_FMA>(macros, a, block, variant, s);
-    case PLB_FP32: return launch_prec<PLB_FP32>(macros, a, block, variant, s);
-    case PLB_FP16DEV: return launch_prec<PLB_FP16DEV>(macros, a, block, variant, s);
-    case PLB_BF16DEV: return launch_prec<PLB_BF16DEV>(macros, a, block, variant, s);
+    case PLB_FP64_EXACT: return launch_prec<PLB_FP64_EXACT>(macros, a, l, s);
+    case PLB_FP64: return launch_prec<PLB_FP64>(macros, a, l, s);
+    case PLB_FP64_FMA: return launch_prec<PLB_FP64_FMA>(macros, a, l, s);
+    case PLB_FP32: return launch_prec<PLB_FP32>(macros, a, l, s);
+    case PLB_FP16DEV: return launch_prec<PLB_FP16DEV>(macros, a, l, s);
+    case PLB_BF16DEV: return launch_prec<PLB_BF16DEV>(macros, a, l, s);
     default: return cudaErrorInvalidValue;
     }
 }

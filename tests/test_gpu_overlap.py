@@ -1,8 +1,8 @@
 """Steps of one call overlap each other on the device (a step's CTAs start
 while the step before drains).  One call of many steps and the same steps
 one call at a time, each waited for, have to give the same bits: at the
-sizes where the default CTA changes (one CTA per SM still covers the domain
-with half the threads) and on both sides of the number of waves up to which
+sizes where the default CTA changes, where the grid is spread over the SMs
+(less than one wave), and on both sides of the number of waves up to which
 the neighbour words are loaded before the wait."""
 import numpy as np
 import pytest
@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
     ("fp64_exact", (9, 8, 7)), ("fp64_exact", (24, 31, 33)), ("fp64_exact", (37, 36, 41)),
     ("fp64_exact", (161, 160, 162)), ("fp64_exact", (166, 165, 167)),
     ("fp64", (30, 31, 31)), ("fp64", (108, 110, 111)), ("fp64", (112, 113, 114)),
-    ("fp64_fma", (31, 30, 30)), ("fp32", (29, 31, 30)), ("fp32", (222, 221, 222)),
+    ("fp64_fma", (31, 30, 30)), ("fp64_exact", (60, 61, 59)), ("fp64", (36, 38, 37)),
+    ("fp64_fma", (44, 43, 45)), ("fp32", (72, 71, 72)), ("fp16dev", (36, 36, 35)), ("fp32", (29, 31, 30)), ("fp32", (222, 221, 222)),
     ("fp32", (226, 225, 226)), ("fp16dev", (40, 41, 39)), ("bf16dev", (228, 226, 227))])
 def test_one_call_equals_waited_steps(precision, dims):
     steps = 7
