@@ -42,7 +42,7 @@ BYTES_PER_NODE = {"fp64_exact": 376, "fp64": 376, "fp64_fma": 376, "fp32": 224,
 # step-kernel sources it was captured from.  A record is reported only
 # while the kernel sources are unchanged.
 PROFILES = os.path.join(ROOT, "profiles")
-STEP_SOURCES = ("plb_step.cu", "plb_fx.h", "plb_emu.h", "plb_internal.h")
+STEP_SOURCES = ("plb_step.cu", "plb_fx.h", "plb_ex.h", "plb_emu.h", "plb_internal.h")
 
 
 def source_digest():

@@ -2,8 +2,9 @@
  * plb_emu.h - IEEE-754 double multiply, round to nearest even, on the
  * integer pipes.
  *
- * The bit-exact FP64 collision spends its time on GB300's FP64 pipe (about
- * 2 operations per clock per SM).  Part of its multiplies run here instead,
+ * GB300's FP64 pipe makes about 2 operations per clock per SM.  Where the
+ * bit-exact FP64 collision leaves the domain of its integer form (plb_ex.h),
+ * part of its multiplies run here instead,
  * on the integer multiply-add pipe, and return the same bits as the FP64
  * pipe: the 106-bit product of the two 53-bit significands is formed
  * exactly and rounded once, to nearest, ties to even.  (An add done the same

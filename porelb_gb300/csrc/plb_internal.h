@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "porelb_gpu.h"
+#include "plb_ex.h"
 #include "plb_fx.h"
 
 /* Every device allocation of the library goes through here, so that a test
@@ -75,6 +76,7 @@ struct Coeffs {
     float omega_f, om1_f, c_f, half_force_f;
     float scale, inv_scale; /* deviation storage scale */
     fx::Consts fxk;         /* fixed-point form */
+    ex_::Consts exk;        /* bit-exact form */
     int it;                 /* iteration number (the it > 0 rule) */
     /* bit-exact form: a run constant outside the range of the integer
      * multiply's node check (every node then takes the native multiply) */

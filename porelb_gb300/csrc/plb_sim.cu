@@ -230,6 +230,7 @@ void make_coeffs(double tau, double force, float scale, Coeffs *c)
     c->scale = scale;
     c->inv_scale = 1.0f / scale;
     c->fxk = fx::make_consts(tau, force);
+    c->exk = ex_::make_consts(c->omega, c->om1, c->k3, c->force, c->half_force);
     const double consts[5] = {c->omega, c->om1, c->k3, c->force, c->half_force};
     for (double x : consts) {
         uint64_t b;

@@ -13,7 +13,9 @@
  *
  * Forms:
  *   FP64_EXACT  the reference's operations in the reference's order with
- *               round-to-nearest intrinsics (no FMA contraction): bit-exact.
+ *               one rounding each: bit-exact.  Most of them run on the
+ *               integer pipes (plb_ex.h), the rest and the nodes outside its
+ *               domain with round-to-nearest intrinsics.
  *   FP64        exact Q60 fixed-point collision on the integer pipes
  *               (plb_fx.h); nodes outside its range fall back to FP64_FMA.
  *   FP64_FMA    the same algebra in native FP64, restructured for FMA.
@@ -25,6 +27,7 @@
 #include <string.h>
 
 #include "plb_emu.h"
+#include "plb_ex.h"
 #include "plb_internal.h"
 
 namespace plb {
@@ -44,9 +47,10 @@ __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a,
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 /* the same product on the integer pipes (plb_emu.h): the same bits for a
  * node whose values, density and run constants passed the range check.
- * The bit-exact collision sends 84 of its 97 products per node here, which
- * balances the FP64 and integer pipes (2.05 -> 2.68 GLUPS at 256^3); a
- * node outside the range takes the NATIVE products. */
+ * The bit-exact collision outside plb_ex.h's domain sends 84 of its 97
+ * products per node here, which balances the FP64 and integer pipes (2.05 ->
+ * 2.68 GLUPS at 256^3); a node outside this range too takes the NATIVE
+ * products. */
 template <bool NATIVE>
 __device__ __forceinline__ double imul(double a, double b)
 {
@@ -399,42 +403,83 @@ template <> struct StoreOf<PLB_BF16DEV> { using T = __nv_bfloat16; };
  * by kernel variant (0 = default; 1 and 3 the alternatives the launch tuner
  * tries): fixed-point FP64 128 / 80 / 64 registers, the FP32 and 16-bit
  * forms 48 / unconstrained / 40 registers (48 is the faster on GB300: FP16
- * deviations 39.1 against 38.4 GLUPS at 512^3), the other FP64 forms
- * unconstrained. */
+ * deviations 39.1 against 38.4 GLUPS at 512^3), bit-exact FP64 80 (its
+ * integer chains wait on themselves, so warps pay: 5.8 GLUPS at 256^3
+ * against 4.9 with 108 registers and 16 warps per SM; 64 registers spill:
+ * 5.7), FMA FP64 unconstrained. */
 template <int PREC, int V> struct MinBlocks {
     static constexpr bool dev = PREC == PLB_FP32 || PREC == PLB_FP16DEV || PREC == PLB_BF16DEV;
     static constexpr int v = PREC == PLB_FP64 ? (V == 1 ? 3 : V == 3 ? 4 : 2)
                            : dev ? (V == 1 ? 1 : V == 3 ? 6 : 5)
-                                 : 1;
+                         : PREC == PLB_FP64_EXACT ? 3 : 1;
 };
 
-/* Gather, collide and store node i.  Returns the macros; *dev_max receives
- * the largest stored deviation magnitude of the 16-bit forms. */
-/* The bit-exact collision of node i with every product on the FP64 pipe,
- * from its streamed values gathered again, stored: the path of a node
- * whose values or density (or the run's constants) lie outside the range
- * of the integer multiply's check, such as an infinity, a NaN, a subnormal
- * or an extreme value.  Out of line, so the common path keeps its
+/* The bit-exact collision of node i outside plb_ex.h's common domain, from
+ * its streamed values gathered again, stored: plb_ex.h's form for tau within
+ * 1/16 of 1; else the products on the integer pipes for a node in their
+ * range, every product on the FP64 pipe for one whose values or density (or
+ * the run's constants) lie outside it, such as an infinity, a NaN, a
+ * subnormal or an extreme value.  Out of line, so the common path keeps its
  * registers. */
-__device__ __noinline__ Macro exact_node_native(const double *fin, double *fout,
-                                                const uint32_t *nbr, long long np,
-                                                long long i, const Coeffs &co)
+__device__ __noinline__ Macro exact_node_wide(const double *fin, double *fout,
+                                              const uint32_t *nbr, long long np,
+                                              long long i, const Coeffs *run, int it,
+                                              unsigned int *flags)
 {
+    Coeffs co = *run;
+    co.it = it;
     double raw[Q];
     gather<double>(fin, nbr, np, i, raw);
-    uint32_t unused = 0;
-    const Macro m = collide_fp64_exact<true>(raw, co, unused);
+    Macro m;
+    uint32_t outside = co.exk.ok ^ 2u;
+    if (!outside) {
+        uint64_t b[Q];
+#pragma unroll
+        for (int j = 0; j < Q; j++) b[j] = (uint64_t)__double_as_longlong(raw[j]);
+        ex_::Out o;
+        outside = ex_::collide<true>(b, co.exk, co.it > 0, o, [&](int j, uint64_t v) {
+            __stcs(fout + (long long)j * np + i, __longlong_as_double((long long)v));
+        });
+        if (!outside) {
+            m.rho = o.rho; m.u = o.u; m.v = o.v; m.w = o.w;
+            m.bad = o.bad != 0u;
+            return m;
+        }
+    }
+    /* the integer multiply needs the node's values in [2^-64, 2^64) (and its
+     * density, checked in the collision): their smallest and largest exponent
+     * field (a zero value, which the range admits but a distribution never
+     * is, takes the native path) */
+    uint32_t emin = 0x7ffu, emax = 0u;
+#pragma unroll
+    for (int j = 0; j < Q; j++) {
+        const uint32_t e = ((uint32_t)__double2hiint(raw[j]) >> 20) & 0x7ffu;
+        emin = min(emin, e);
+        emax = max(emax, e);
+    }
+    outside = (uint32_t)co.exact_native | (uint32_t)(emin < 1023u - 64u) |
+              (uint32_t)(emax > 1023u + 63u);
+    if (!outside) m = collide_fp64_exact<false>(raw, co, outside);
+    if (outside) {
+        *flags |= 2u;
+        gather<double>(fin, nbr, np, i, raw);
+        uint32_t unused = 0;
+        m = collide_fp64_exact<true>(raw, co, unused);
+    }
 #pragma unroll
     for (int j = 0; j < Q; j++) __stcs(fout + (long long)j * np + i, raw[j]);
     return m;
 }
 
-/* Collide node i's streamed values raw[] and store them. */
+/* Collide node i's streamed values raw[] and store them.  run: co in global
+ * or parameter memory (its iteration number may be another's), for the path
+ * that is out of line. */
 template <int PREC, bool MACRO, typename T>
 __device__ __forceinline__ Macro collide_node(T (&raw)[Q], const T *fin, T *fout,
                                               const uint32_t *nbr, long long np,
                                               long long i, const Coeffs &co,
-                                              unsigned int &flags, float &dev_max)
+                                              const Coeffs *run, unsigned int &flags,
+                                              float &dev_max)
 {
     Macro m;
     if constexpr (PREC == PLB_FP64) {
@@ -449,29 +494,22 @@ __device__ __forceinline__ Macro collide_node(T (&raw)[Q], const T *fin, T *fout
         }
 #pragma unroll
         for (int j = 0; j < Q; j++) __stcs(fout + (long long)j * np + i, raw[j]);
-    } else if constexpr (PREC == PLB_FP64_EXACT || PREC == PLB_FP64_FMA) {
-        if constexpr (PREC == PLB_FP64_EXACT) {
-            /* the integer multiply needs the node's values in [2^-64, 2^64)
-             * (and its density, checked in the collision): their smallest
-             * and largest exponent field (a zero value, which the range
-             * admits but a distribution never is, takes the native path) */
-            uint32_t emin = 0x7ffu, emax = 0u;
+    } else if constexpr (PREC == PLB_FP64_EXACT) {
+        uint64_t b[Q];
 #pragma unroll
-            for (int j = 0; j < Q; j++) {
-                const uint32_t e = ((uint32_t)__double2hiint(raw[j]) >> 20) & 0x7ffu;
-                emin = min(emin, e);
-                emax = max(emax, e);
-            }
-            uint32_t outside = (uint32_t)co.exact_native | (uint32_t)(emin < 1023u - 64u) |
-                               (uint32_t)(emax > 1023u + 63u);
-            if (!outside) m = collide_fp64_exact<false>(raw, co, outside);
-            if (outside) {
-                flags |= 2u;
-                return exact_node_native(fin, fout, nbr, np, i, co);
-            }
-        } else {
-            m = collide_fp64_fma(raw, co);
-        }
+        for (int j = 0; j < Q; j++) b[j] = (uint64_t)__double_as_longlong(raw[j]);
+        ex_::Out o;
+        uint32_t outside = co.exk.ok ^ 1u;
+        if (!outside)
+            outside = ex_::collide<false>(b, co.exk, co.it > 0, o, [&](int j, uint64_t v) {
+                __stcs(fout + (long long)j * np + i, __longlong_as_double((long long)v));
+            });
+        /* it stores all 19 values again */
+        if (outside) return exact_node_wide(fin, fout, nbr, np, i, run, co.it, &flags);
+        m.rho = o.rho; m.u = o.u; m.v = o.v; m.w = o.w;
+        m.bad = o.bad != 0u;
+    } else if constexpr (PREC == PLB_FP64_FMA) {
+        m = collide_fp64_fma(raw, co);
 #pragma unroll
         for (int j = 0; j < Q; j++) __stcs(fout + (long long)j * np + i, raw[j]);
     } else {
@@ -550,7 +588,7 @@ k_step(const StepArgs a)
         float dm = 0.f;
         unsigned int fl = 0;
         const Macro m = collide_node<PREC, MACRO>(raw, (const T *)a.fin, (T *)a.fout, a.nbr,
-                                                  a.npad, i, a.co, fl, dm);
+                                                  a.npad, i, a.co, &a.co, fl, dm);
         if (fl) atomicOr(a.flags, fl);
         if (m.bad) {
             const unsigned long long key =
@@ -640,7 +678,7 @@ k_batch_step(const BatchArgs a)
             co.it = *a.t_base + a.t_off - sp->start;
             unsigned int fl = 0;
             const Macro m = collide_node<PREC, MACRO>(raw, (const T *)a.fin, (T *)a.fout,
-                                                      a.nbr, a.npad, i, co, fl, dmax);
+                                                      a.nbr, a.npad, i, co, &sp->co, fl, dmax);
             if (fl | (m.bad ? 4u : 0u)) atomicOr(a.serr + s, fl | (m.bad ? 4u : 0u));
             if (MACRO) {
                 const long long np = a.npad;
@@ -812,11 +850,13 @@ void plan_step(int precision, int n, StepLaunch *l)
 }
 
 /* Threads per CTA of the plain step.  128 for the fixed-point and FMA FP64
- * forms; 256 for the others once 128-thread CTAs fill the device (FP16 at
- * 22M nodes 575 against 648 us), and 128 below, where the finer grain
- * spreads better (FP32 at 131k nodes 3.8 against 4.2 us).  Domains that 64-thread CTAs cover with one
+ * forms; 256 for the others once 128-thread CTAs fill the device, since
+ * warps of one CTA share instruction fetches (bit-exact form 1019 against
+ * 1103 us at 256^3, FP16 at 22M nodes 575 against 648), and 128 below, where the finer grain
+ * spreads better (bit-exact at 92k nodes 20.7 against 23.8 us, FP32 at 76k
+ * 2.8 / 2.7, at 131k 3.8 / 4.2).  Domains that 64-thread CTAs cover with one
  * per SM take those: fewer warps share an SM's pipes (1.4k-9k nodes: FMA 7.0
- * against 7.7 us, FP64 2.8 / 3.1). */
+ * against 7.7 us, FP64 2.8 / 3.1, bit-exact 9.4 / 9.8). */
 template <int PREC>
 static int block_prec(int n)
 {
