@@ -194,15 +194,18 @@ __global__ void k_translate_words(const uint32_t *src, long long snp, long long 
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
+    uint32_t words[Q - 1];
+#pragma unroll
     for (int j = 1; j < Q; j++) {
-        const uint32_t w = src[(long long)(j - 1) * snp + sbase + k];
+        const uint32_t w = src[word_at(j, sbase + k, snp)];
         uint32_t o;
         if (w == srest) o = drest;
         else if ((long long)(uint32_t)(w - (uint32_t)sbase) < (long long)n)
             o = (uint32_t)(dbase + (long long)(w - (uint32_t)sbase));
         else o = bounce_word(j, dbase + k, dnp);
-        dst[(long long)(j - 1) * dnp + dbase + k] = o;
+        words[j - 1] = o;
     }
+    store_words(dst, dnp, dbase + k, words);
 }
 
 /* a sample's stored deviations moved into another storage form: g =
@@ -543,7 +546,7 @@ static int add_dflag(plb_batch *b, const uint8_t *dflag, int nx, int ny, int nz,
                               ? plb_auto_ordering(n, nz, (int)b->elem, b->device)
                               : b->ordering;
         rc = flag_tables(dflag, nx, ny, nz, 1, order, 0, 0, lexbits, lexoffs, n,
-                         b->npad, b->perm + base, b->coord + base, b->nbr + base,
+                         b->npad, b->perm + base, b->coord + base, b->nbr,
                          (uint32_t)base, (uint32_t)b->rest, b->adm);
         if (rc != PLB_OK) free_range(b, blk0, nblk);
     }

@@ -125,6 +125,7 @@ __global__ void k_nbr_from_flag(const uint32_t *lexbits, const uint32_t *obits,
     if (k >= n) return;
     const int x = coord[k], y = coord[npad + k], z = coord[2 * npad + k];
     const size_t cx = ((size_t)z * g.ny + y) * g.nx + x;
+    uint32_t words[Q - 1];
 #pragma unroll
     for (int j = 1; j < Q; j++) {
         int sx = x - ex(j), sy = y - ey(j), sz = z - ez(j);
@@ -150,8 +151,9 @@ __global__ void k_nbr_from_flag(const uint32_t *lexbits, const uint32_t *obits,
             word = bounce_word(j, (long long)word_base + k, npad);
         else
             word = rest_word;
-        nbr[(long long)(j - 1) * npad + k] = word;
+        words[j - 1] = word;
     }
+    store_words(nbr, npad, (long long)word_base + k, words);
 }
 
 /* --------------------------------------------------------- sphere pack */

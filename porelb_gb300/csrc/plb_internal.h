@@ -63,6 +63,28 @@ __host__ __device__ constexpr int wclass(int j)
  * 2 * npad < 2^31, hence kMaxNodes. */
 constexpr long long kMaxNodes = (1LL << 30) - 512;
 
+/* The 18 words of a node lie in five rows, four of four words and one of
+ * two, so that a thread reads them with four 16-byte loads and one 8-byte
+ * load: where word j of node i is. */
+__host__ __device__ constexpr long long word_at(int j, long long i, long long npad)
+{
+    return j <= 16 ? (long long)((j - 1) & ~3) * npad + 4 * i + ((j - 1) & 3)
+                   : 16 * npad + 2 * i + (j - 17);
+}
+
+#if defined(__CUDACC__)
+/* store the words w[j - 1] of node i */
+__device__ __forceinline__ void store_words(uint32_t *nbr, long long npad, long long i,
+                                            const uint32_t (&w)[18])
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        *(uint4 *)(nbr + word_at(4 * q + 1, i, npad)) =
+            make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+    *(uint2 *)(nbr + word_at(17, i, npad)) = make_uint2(w[16], w[17]);
+}
+#endif
+
 __host__ __device__ inline uint32_t bounce_word(int j, long long i, long long npad)
 {
     return (uint32_t)(i + (long long)(opp(j) - j) * npad);
@@ -86,7 +108,7 @@ struct Coeffs {
 struct StepArgs {
     const void *fin;
     void *fout;
-    const uint32_t *nbr;  /* [18][npad] */
+    const uint32_t *nbr;  /* word_at() */
     const int *perm;      /* new -> reference index (density guard report) */
     long long npad;
     int n;
@@ -102,14 +124,18 @@ struct StepArgs {
 };
 
 /* Waves of resident CTAs up to which a step loads its words before it waits
- * for the step before; above it, each gather goes out as its word arrives.
+ * for the step before; above it, the gathers go out as their words arrive.
  * In a short launch most CTAs start while the step before still drains, and
- * their word loads then cost nothing (FP32: 3.3 against 3.9 us at 92k nodes,
- * 6.8 against 7.3 at 310k; FP16 19.4 against 20.4 at 734k).  In a long one
- * few do, and 18 words held before the first gather make the loads burstier
- * (fixed-point FP64: 48.0 against 47.1 us at 734k nodes, 9 waves, 2% at 22M;
- * FP32 and 16-bit: even at 30 waves, 2% slower at 115). */
-constexpr int words_first_waves(int precision) { return precision == PLB_FP64 ? 6 : 20; }
+ * their word loads then cost nothing.  In a long one few do, and 18 words
+ * held before the first gather cost registers and make the loads burstier
+ * (FP32, words first / after: 3.2 / 3.4 us at 92k nodes, 7.0 / 6.7 at 310k;
+ * FP16 2.75 / 3.3, 41.2 / 38.6 at 1.4M; fixed-point FP64 24.2 / 24.8 at 310k,
+ * 48.0 / 47.1 at 734k, 9 waves). */
+constexpr int words_first_waves(int precision)
+{
+    return precision == PLB_FP64 ? 6
+         : precision == PLB_FP64_EXACT || precision == PLB_FP64_FMA ? 20 : 1;
+}
 
 /* One sample of a batch (device copy). */
 struct SampleDev {

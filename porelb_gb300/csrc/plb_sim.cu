@@ -370,6 +370,7 @@ __global__ void k_build_nbr(const plb_node_info *V, const int *perm,
     coord[k] = r.x;
     coord[npad + k] = r.y;
     coord[2 * npad + k] = r.z;
+    uint32_t words[Q - 1];
 #pragma unroll
     for (int j = 1; j < Q; j++) {
         const plb_neighbor_info sn = r.nb_info[opp(j) - 1];
@@ -405,8 +406,9 @@ __global__ void k_build_nbr(const plb_node_info *V, const int *perm,
             word = bounce_word(j, k, npad);
         else
             word = (uint32_t)n;
-        nbr[(long long)(j - 1) * npad + k] = word;
+        words[j - 1] = word;
     }
+    store_words(nbr, npad, k, words);
 }
 
 /* --------------------------------------------------------- state kernels */
@@ -493,7 +495,7 @@ __global__ void k_get_streamed(const T *f, const uint32_t *nbr, const int *perm,
     const long long o = (long long)perm[k] * Q;
 #pragma unroll
     for (int j = 0; j < Q; j++) {
-        const long long at = j == 0 ? k : (long long)j * npad + (int)nbr[(j - 1) * npad + k];
+        const long long at = j == 0 ? k : (long long)j * npad + (int)nbr[word_at(j, k, npad)];
         if constexpr (sizeof(T) == 8) {
             out[o + j] = ((const double *)f)[at];
         } else {

@@ -84,7 +84,16 @@ __device__ __forceinline__ void load_words(const uint32_t *nbr, long long np, lo
                                            int (&w)[Q - 1])
 {
 #pragma unroll
-    for (int j = 0; j < Q - 1; j++) w[j] = (int)__ldg(nbr + (long long)j * np + i);
+    for (int q = 0; q < 4; q++) {
+        const int4 v = __ldg((const int4 *)(nbr + word_at(4 * q + 1, i, np)));
+        w[4 * q] = v.x;
+        w[4 * q + 1] = v.y;
+        w[4 * q + 2] = v.z;
+        w[4 * q + 3] = v.w;
+    }
+    const int2 v = __ldg((const int2 *)(nbr + word_at(17, i, np)));
+    w[16] = v.x;
+    w[17] = v.y;
 }
 
 template <typename T>
@@ -96,17 +105,14 @@ __device__ __forceinline__ void gather_words(const T *fin, long long np, long lo
     for (int j = 1; j < Q; j++) f[j] = fin[(long long)j * np + w[j - 1]];
 }
 
-/* the same two in one: each gather goes out as its word arrives */
+/* the same two in one: the gathers go out as their words arrive */
 template <typename T>
 __device__ __forceinline__ void gather(const T *fin, const uint32_t *nbr,
                                        long long np, long long i, T (&f)[Q])
 {
-    f[0] = fin[i];
-#pragma unroll
-    for (int j = 1; j < Q; j++) {
-        const int w = (int)__ldg(nbr + (long long)(j - 1) * np + i);
-        f[j] = fin[(long long)j * np + w];
-    }
+    int w[Q - 1];
+    load_words(nbr, np, i, w);
+    gather_words<T>(fin, np, i, w, f);
 }
 
 /* The streamed values of node i (if valid), after the step before: WF loads
@@ -403,14 +409,16 @@ template <> struct StoreOf<PLB_BF16DEV> { using T = __nv_bfloat16; };
  * by kernel variant (0 = default; 1 and 3 the alternatives the launch tuner
  * tries): fixed-point FP64 128 / 80 / 64 registers, the FP32 and 16-bit
  * forms 48 / unconstrained / 40 registers (48 is the faster on GB300: FP16
- * deviations 39.1 against 38.4 GLUPS at 512^3), bit-exact FP64 80 (its
+ * deviations 39.1 against 38.4 GLUPS at 512^3) or, with the words held before
+ * the wait, 64 (at 48 they spill: FP16 at 92k nodes 2.94 against 2.75 us),
+ * bit-exact FP64 80 (its
  * integer chains wait on themselves, so warps pay: 5.8 GLUPS at 256^3
  * against 4.9 with 108 registers and 16 warps per SM; 64 registers spill:
  * 5.7), FMA FP64 unconstrained. */
-template <int PREC, int V> struct MinBlocks {
+template <int PREC, int V, bool WF> struct MinBlocks {
     static constexpr bool dev = PREC == PLB_FP32 || PREC == PLB_FP16DEV || PREC == PLB_BF16DEV;
     static constexpr int v = PREC == PLB_FP64 ? (V == 1 ? 3 : V == 3 ? 4 : 2)
-                           : dev ? (V == 1 ? 1 : V == 3 ? 6 : 5)
+                           : dev ? (V == 1 ? 1 : V == 3 ? 6 : WF ? 4 : 5)
                          : PREC == PLB_FP64_EXACT ? 3 : 1;
 };
 
@@ -539,7 +547,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes)
 
 /* Thread 0 of a block asks L2 for the node range of block b (a block that
  * starts some time after this one, pf_blocks blocks later in launch order):
- * its 18 rows of neighbour words and its 19 rows of distributions.  In
+ * its five rows of neighbour words and its 19 rows of distributions.  In
  * Morton order most gathers of that block read inside the ranges of the
  * blocks launched near it, so its loads then wait for L2 instead of DRAM.  Rows are npad elements (a
  * multiple of 64) and the block size is a multiple of 32, so every range
@@ -552,16 +560,16 @@ __device__ __forceinline__ void prefetch_block(const T *fin, const uint32_t *nbr
     const long long i0 = b * bs;
     if (i0 >= n) return;
     const long long cnt = np - i0 < bs ? np - i0 : bs;
-    const unsigned wb = (unsigned)(cnt * 4);
     const unsigned fb = (unsigned)(cnt * (long long)sizeof(T));
 #pragma unroll 1
-    for (int j = 0; j < Q - 1; j++) prefetch_l2(nbr + (long long)j * np + i0, wb);
+    for (int j = 1; j < 17; j += 4) prefetch_l2(nbr + word_at(j, i0, np), (unsigned)(cnt * 16));
+    prefetch_l2(nbr + word_at(17, i0, np), (unsigned)(cnt * 8));
 #pragma unroll 1
     for (int j = 0; j < Q; j++) prefetch_l2(fin + (long long)j * np + i0, fb);
 }
 
 template <int PREC, bool MACRO, int VARIANT, bool WF>
-__global__ void __launch_bounds__(256, MinBlocks<PREC, VARIANT>::v)
+__global__ void __launch_bounds__(256, MinBlocks<PREC, VARIANT, WF>::v)
 k_step(const StepArgs a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -632,7 +640,7 @@ k_step(const StepArgs a)
  * order their gathers share L2 lines (a fixed grid looping over the list
  * lost that and ran 23% slower in the FP64 form). */
 template <int PREC, bool MACRO, int BT, bool WF>
-__global__ void __launch_bounds__(BT, MinBlocks<PREC, 0>::v * (kBatchBlock / BT))
+__global__ void __launch_bounds__(BT, MinBlocks<PREC, 0, WF>::v * (kBatchBlock / BT))
 k_batch_step(const BatchArgs a)
 {
     using T = typename StoreOf<PREC>::T;
@@ -918,7 +926,7 @@ int batch_wave_blocks(int precision, int cta)
 template <int PREC, int BT>
 static const void *batch_fn(bool macros, bool wf)
 {
-    if constexpr (PREC == PLB_FP16DEV || PREC == PLB_BF16DEV) {
+    if constexpr (MinBlocks<PREC, 0, true>::dev) {
         if (!wf)
             return macros ? (const void *)k_batch_step<PREC, true, BT, false>
                           : (const void *)k_batch_step<PREC, false, BT, false>;
@@ -927,10 +935,10 @@ static const void *batch_fn(bool macros, bool wf)
                   : (const void *)k_batch_step<PREC, false, BT, true>;
 }
 
-/* The pool's words come first in every launch of the forms of 4 and 8 bytes
- * (pools of 0.1M to 6M nodes: FP64 3-6% faster than words after the wait,
- * FP32 even to 10%); the 16-bit forms', up to the same number of waves as a
- * plain step's (0.1M nodes 3.2 against 3.6 us, 5M nodes 132 against 130). */
+/* The pool's words come first in every launch of the FP64 forms (0.1M to 6M
+ * nodes: 3-6% faster than words after the wait); the deviation forms', up to
+ * the same number of waves as a plain step's (FP32 92k nodes 3.6 against 3.9
+ * us, 5M nodes 171 against 162). */
 template <int PREC>
 static const void *batch_fn_cta(bool macros, int cta, int grid)
 {
