@@ -1235,6 +1235,7 @@ int plb_batch_get_f(plb_batch *b, int id, double *f_aos)
             k_get_f_sample<__nv_bfloat16><<<gb(h.n, B), B, 0, b->st>>>((const __nv_bfloat16 *)f, b->npad, base, h.n, b->perm, inv, d);
     }
     cudaError_t e = cudaGetLastError();
+    host_populate(f_aos, bytes);
     if (e == cudaSuccess) e = cudaMemcpyAsync(f_aos, d, bytes, cudaMemcpyDeviceToHost, b->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
     cudaFree(d);
@@ -1256,6 +1257,7 @@ int plb_batch_get_macros(plb_batch *b, int id, double *rho, double *ux,
                                                    b->perm, d);
     double *dst[4] = {rho, ux, uy, uz};
     cudaError_t e = cudaGetLastError();
+    for (int c = 0; c < 4; c++) host_populate(dst[c], 8 * (size_t)h.n);
     for (int c = 0; c < 4 && e == cudaSuccess; c++)
         if (dst[c])
             e = cudaMemcpyAsync(dst[c], d + (size_t)c * h.n, 8 * (size_t)h.n,

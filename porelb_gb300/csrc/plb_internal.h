@@ -169,6 +169,10 @@ struct BatchArgs {
     const int *grp_cur;
 };
 
+/* Make the pages of a host buffer that a device copy is about to write
+ * present (plb_sim.cu). */
+void host_populate(void *p, size_t bytes);
+
 /* Exclusive scan of m uint32 counts into offs (device memory). */
 int scan_words(const uint32_t *cnt, uint32_t *offs, size_t m, cudaStream_t st);
 
