@@ -517,23 +517,17 @@ static void activate(plb_batch *b, int sid)
     b->list_dirty = true;
 }
 
-/* Admit a sample whose flag grid is on the device. */
-static int add_dflag(plb_batch *b, const uint8_t *dflag, int nx, int ny, int nz,
+/* Admit a sample whose flag grid is in w. */
+static int add_dflag(plb_batch *b, const GeomWork &w, int nx, int ny, int nz,
                      const plb_sample_params *sp, int *id)
 {
     int sid = -1;
     for (int k = 0; k < b->max_samples; k++)
         if (!b->s[k].used) { sid = k; break; }
     if (sid < 0) return PLB_ERR_NOMEM;
-    const size_t cells = (size_t)nx * ny * nz;
-    const size_t words = (cells + 31) / 32;
-    uint32_t *lexbits = nullptr, *lexoffs = nullptr;
-    int n = 0, slab0 = 0, rc = PLB_OK;
+    int n = 0, slab0 = 0;
     long long blk0 = -1, nblk = 0;
-    if (plb_cuda_malloc(&lexbits, words * 4) != cudaSuccess ||
-        plb_cuda_malloc(&lexoffs, words * 4) != cudaSuccess)
-        rc = PLB_ERR_NOMEM;
-    if (rc == PLB_OK) rc = flag_rank(dflag, nx, ny, nz, 1, lexbits, lexoffs, &n, &slab0, b->adm);
+    int rc = flag_rank(w, nx, ny, nz, 1, &n, &slab0, b->adm);
     if (rc == PLB_OK) {
         nblk = (n + B - 1) / B;
         if (nblk == 0) nblk = 1;
@@ -545,13 +539,10 @@ static int add_dflag(plb_batch *b, const uint8_t *dflag, int nx, int ny, int nz,
         const int order = b->ordering == PLB_ORDER_AUTO
                               ? plb_auto_ordering(n, nz, (int)b->elem, b->device)
                               : b->ordering;
-        rc = flag_tables(dflag, nx, ny, nz, 1, order, 0, 0, lexbits, lexoffs, n,
-                         b->npad, b->perm + base, b->coord + base, b->nbr,
-                         (uint32_t)base, (uint32_t)b->rest, b->adm);
+        rc = flag_tables(w, nx, ny, nz, 1, order, 0, 0, n, b->npad, b->perm + base, b->coord + base,
+                         b->nbr, (uint32_t)base, (uint32_t)b->rest, b->adm);
         if (rc != PLB_OK) free_range(b, blk0, nblk);
     }
-    cudaFree(lexbits);
-    cudaFree(lexoffs);
     if (rc != PLB_OK) return rc;
 
     SampleHost &h = b->s[sid];
@@ -606,14 +597,14 @@ int plb_batch_add_flag(plb_batch *b, const uint8_t *flag, int nx, int ny, int nz
         return PLB_ERR_ARG;
     BCK(cudaSetDevice(b->device));
     const size_t cells = (size_t)nx * ny * nz;
-    uint8_t *d = nullptr;
-    BCK(plb_cuda_malloc(&d, cells));
-    int rc = PLB_OK;
-    if (cudaMemcpyAsync(d, flag, cells, cudaMemcpyHostToDevice, b->adm) != cudaSuccess)
+    GeomWork w;
+    int rc = geom_alloc(&w, nx, ny, nz, 1);
+    if (rc == PLB_OK &&
+        cudaMemcpyAsync(w.flag, flag, cells, cudaMemcpyHostToDevice, b->adm) != cudaSuccess)
         rc = PLB_ERR_CUDA;
-    if (rc == PLB_OK) rc = add_dflag(b, d, nx, ny, nz, sp, id);
+    if (rc == PLB_OK) rc = add_dflag(b, w, nx, ny, nz, sp, id);
     cudaStreamSynchronize(b->adm);
-    cudaFree(d);
+    geom_free(&w);
     return rc;
 }
 
@@ -627,14 +618,14 @@ int plb_batch_add_packed(plb_batch *b, uint64_t seed, int nx, int ny, int nz,
         !(porosity >= 0.0) || !(porosity <= 1.0))
         return PLB_ERR_ARG;
     BCK(cudaSetDevice(b->device));
-    const size_t cells = (size_t)nx * ny * nz;
-    uint8_t *d = nullptr;
-    BCK(plb_cuda_malloc(&d, cells));
-    int rc = sphere_pack_device(seed, nx, ny, nz, rmin, rmax, porosity, d, num_spheres,
+    GeomWork w;
+    int rc = geom_alloc(&w, nx, ny, nz, 1);
+    if (rc == PLB_OK)
+        rc = sphere_pack_device(seed, nx, ny, nz, rmin, rmax, porosity, w.flag, num_spheres,
                                 porosity_out, b->adm);
-    if (rc == PLB_OK) rc = add_dflag(b, d, nx, ny, nz, sp, id);
+    if (rc == PLB_OK) rc = add_dflag(b, w, nx, ny, nz, sp, id);
     cudaStreamSynchronize(b->adm);
-    cudaFree(d);
+    geom_free(&w);
     return rc;
 }
 

@@ -12,7 +12,10 @@
  * 152-byte-per-node V.bin records.  For a flag with values 0/1 the result is
  * identical to plb_create on the table plb_build_table writes.
  */
+#include <math.h>
 #include <stdio.h>
+#include <stdlib.h>
+#include <string.h>
 
 #include "plb_internal.h"
 
@@ -20,22 +23,36 @@ namespace plb {
 
 /* ------------------------------------------------------------- bitmaps */
 
-/* lexicographic fluid bitmap: word w covers cells 32w .. 32w+31 */
+/* bits 0..3: the four 0/1 bytes of v */
+__device__ __forceinline__ uint32_t nibble(uint32_t v)
+{
+    return (v * 0x01020408u) >> 24 & 15u;
+}
+
+/* lexicographic fluid bitmap: word w covers cells 32w .. 32w+31 (flag is 16-
+ * byte aligned) */
 __global__ void k_flag_bits(const uint8_t *flag, size_t cells, uint32_t *bits,
                             uint32_t *cnt, size_t words, unsigned *bad)
 {
     const size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= words) return;
-    uint32_t b = 0;
+    uint32_t b = 0, over = 0;
     const size_t c0 = w * 32;
-    for (int k = 0; k < 32; k++) {
-        const size_t c = c0 + k;
-        if (c < cells) {
-            const uint8_t v = flag[c];
-            if (v > 1) atomicOr(bad, 1u);
-            b |= (uint32_t)(v == 1) << k;
+    if (c0 + 32 <= cells) {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const uint4 v = __ldg((const uint4 *)(flag + c0) + q);
+            over |= v.x | v.y | v.z | v.w;
+            b |= (nibble(v.x) | nibble(v.y) << 4 | nibble(v.z) << 8 | nibble(v.w) << 12)
+                 << (16 * q);
+        }
+    } else {
+        for (int k = 0; k < (int)(cells - c0); k++) {
+            over |= flag[c0 + k];
+            b |= (uint32_t)(flag[c0 + k] & 1u) << k;
         }
     }
+    if (over & 0xfefefefeu) atomicOr(bad, 1u);
     bits[w] = b;
     cnt[w] = __popc(b);
 }
@@ -75,8 +92,7 @@ struct Grid {
 
 __device__ __forceinline__ uint64_t device_key(const Grid &g, int x, int y, int z)
 {
-    return g.morton ? morton_code(x, y, z, g.bx, g.by, g.bz)
-                    : ((uint64_t)z * g.ny + y) * g.nx + x;
+    return morton_code(x, y, z, g.bx, g.by, g.bz);
 }
 
 __global__ void k_mark_order(const uint32_t *lexbits, Grid g, size_t cells,
@@ -91,69 +107,121 @@ __global__ void k_mark_order(const uint32_t *lexbits, Grid g, size_t cells,
     atomicOr(obits + (k >> 5), 1u << (k & 31));
 }
 
-/* device index, reference index and coordinates of every fluid cell */
-__global__ void k_assign_from_flag(const uint32_t *lexbits, const uint32_t *lexoffs,
-                                   const uint32_t *obits, const uint32_t *ooffs,
-                                   Grid g, size_t cells, int n, long long npad,
-                                   int *perm, uint16_t *coord)
+/* total fluid cells (meta[0]; meta[1] is the bad-value flag) and the first
+ * node of every z slab (meta[2 ..]) */
+__global__ void k_rank_meta(const uint32_t *bits, const uint32_t *offs, size_t words,
+                            size_t cells, size_t slab_cells, int num_p, uint32_t *meta)
 {
-    const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cells || !bit_at(lexbits, c)) return;
-    const int x = (int)(c % g.nx);
-    const int y = (int)((c / g.nx) % g.ny);
-    const int z = (int)(c / ((size_t)g.nx * g.ny));
-    const uint32_t k = rank_in(obits, ooffs, device_key(g, x, y, z));
-    if (k >= (uint32_t)n) return;
-    perm[k] = (int)rank_in(lexbits, lexoffs, c);
-    coord[k] = (uint16_t)x;
-    coord[npad + k] = (uint16_t)y;
-    coord[2 * npad + k] = (uint16_t)z;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0) meta[0] = offs[words - 1] + __popc(bits[words - 1]);
+    if (p < num_p) {
+        const size_t c = (size_t)p * slab_cells;
+        meta[2 + p] = c < cells ? rank_in(bits, offs, c)
+                                : offs[words - 1] + __popc(bits[words - 1]);
+    }
 }
 
-/* Pull table from the flag: see k_build_nbr for the rule.  s = x - e_j
- * pushes into x if fluid; x bounces if t = x + e_j is solid; when both
- * write, the later in node order wins, i.e. the push iff s's cell index is
- * larger (lexicographic numbering is monotone in the cell index) - or always
- * when s lies in another rank slab and remote_wins is set. */
-__global__ void k_nbr_from_flag(const uint32_t *lexbits, const uint32_t *obits,
-                                const uint32_t *ooffs, Grid g, int slab,
-                                int remote_wins, int halfway, int n, long long npad,
-                                uint32_t word_base, uint32_t rest_word,
-                                const uint16_t *coord, uint32_t *nbr)
+/* What the pull words of one node are made from and go to. */
+struct TableArgs {
+    const uint32_t *lexbits, *lexoffs; /* reference order */
+    const uint32_t *obits, *ooffs;     /* device order (Morton) */
+    Grid g;
+    int slab, remote_wins, halfway, n;
+    long long npad;
+    uint32_t word_base, rest_word;
+    int *perm;
+    uint16_t *coord;
+    uint32_t *nbr;
+};
+
+/* Pull words of the node k on cell (x, y, z): see k_build_nbr for the rule.
+ * s = x - e_j pushes into x if fluid; x bounces if t = x + e_j is solid; when
+ * both write, the later in node order wins, i.e. the push iff s's cell index
+ * is larger (lexicographic numbering is monotone in the cell index) - or
+ * always when s lies in another rank slab and remote_wins is set.  Each of
+ * the 18 neighbours is looked up once, for the direction it sends and the
+ * one it stops. */
+template <bool ROW>
+__device__ __forceinline__ void node_words(const TableArgs &a, int x, int y, int z, size_t cx,
+                                           long long k)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int x = coord[k], y = coord[npad + k], z = coord[2 * npad + k];
-    const size_t cx = ((size_t)z * g.ny + y) * g.nx + x;
+    const Grid &g = a.g;
+    uint32_t idx[Q];
+    uint32_t fluid = 0, later = 0, remote = 0;
+    const int zs = a.remote_wins ? z / a.slab : 0;
+#pragma unroll
+    for (int j = 1; j < Q; j++) {
+        int X = x + ex(j), Y = y + ey(j), Z = z + ez(j);
+        X = X < 0 ? X + g.nx : (X >= g.nx ? X - g.nx : X);
+        Y = Y < 0 ? Y + g.ny : (Y >= g.ny ? Y - g.ny : Y);
+        Z = Z < 0 ? Z + g.nz : (Z >= g.nz ? Z - g.nz : Z);
+        const size_t c = ((size_t)Z * g.ny + Y) * g.nx + X;
+        const uint32_t w = __ldg(a.lexbits + (c >> 5)), bit = 1u << (c & 31);
+        idx[j] = 0;
+        if (w & bit) {
+            fluid |= 1u << j;
+            idx[j] = a.word_base + (ROW ? __ldg(a.lexoffs + (c >> 5)) + __popc(w & (bit - 1u))
+                                        : rank_in(a.obits, a.ooffs, device_key(g, X, Y, Z)));
+        }
+        later |= (uint32_t)(c > cx) << j;
+        if (a.remote_wins) remote |= (uint32_t)(Z / a.slab != zs) << j;
+    }
     uint32_t words[Q - 1];
 #pragma unroll
     for (int j = 1; j < Q; j++) {
-        int sx = x - ex(j), sy = y - ey(j), sz = z - ez(j);
-        int tx = x + ex(j), ty = y + ey(j), tz = z + ez(j);
-        sx = sx < 0 ? sx + g.nx : (sx >= g.nx ? sx - g.nx : sx);
-        sy = sy < 0 ? sy + g.ny : (sy >= g.ny ? sy - g.ny : sy);
-        sz = sz < 0 ? sz + g.nz : (sz >= g.nz ? sz - g.nz : sz);
-        tx = tx < 0 ? tx + g.nx : (tx >= g.nx ? tx - g.nx : tx);
-        ty = ty < 0 ? ty + g.ny : (ty >= g.ny ? ty - g.ny : ty);
-        tz = tz < 0 ? tz + g.nz : (tz >= g.nz ? tz - g.nz : tz);
-        const size_t cs = ((size_t)sz * g.ny + sy) * g.nx + sx;
-        const size_t ct = ((size_t)tz * g.ny + ty) * g.nx + tx;
-        const bool push = bit_at(lexbits, cs);
-        const bool bounce = !bit_at(lexbits, ct);
-        const bool remote = remote_wins && (sz / slab != z / slab);
-        uint32_t word;
-        if (halfway)
-            word = push ? word_base + rank_in(obits, ooffs, device_key(g, sx, sy, sz))
-                        : bounce_word(j, (long long)word_base + k, npad);
-        else if (push && (!bounce || remote || cs > cx))
-            word = word_base + rank_in(obits, ooffs, device_key(g, sx, sy, sz));
-        else if (bounce)
-            word = bounce_word(j, (long long)word_base + k, npad);
-        else
-            word = rest_word;
-        words[j - 1] = word;
+        const int o = opp(j);
+        const bool push = fluid >> o & 1u, bounce = !(fluid >> j & 1u);
+        const bool wins = a.halfway || !bounce || ((later | remote) >> o & 1u);
+        words[j - 1] = push && wins ? idx[o]
+                     : a.halfway || bounce
+                         ? bounce_word(j, (long long)a.word_base + k, a.npad)
+                         : a.rest_word;
     }
-    store_words(nbr, npad, (long long)word_base + k, words);
+    store_words(a.nbr, a.npad, (long long)a.word_base + k, words);
+}
+
+/* x, y, z of a cell */
+__device__ __forceinline__ void cell_xyz(const Grid &g, size_t c, int &x, int &y, int &z)
+{
+    if (c >> 32) {
+        x = (int)(c % g.nx);
+        y = (int)((c / g.nx) % g.ny);
+        z = (int)(c / ((size_t)g.nx * g.ny));
+    } else {
+        const uint32_t r = (uint32_t)c / (uint32_t)g.nx;
+        x = (int)((uint32_t)c - r * (uint32_t)g.nx);
+        z = (int)(r / (uint32_t)g.ny);
+        y = (int)(r - (uint32_t)z * (uint32_t)g.ny);
+    }
+}
+
+/* device index, reference index and coordinates of every fluid cell.  In row
+ * order (ROW) the reference rank is the device index, and no second bitmap
+ * is made. */
+template <bool ROW>
+__global__ void k_assign_from_flag(const TableArgs a, size_t cells)
+{
+    const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= cells || !bit_at(a.lexbits, c)) return;
+    int x, y, z;
+    cell_xyz(a.g, c, x, y, z);
+    const uint32_t i = rank_in(a.lexbits, a.lexoffs, c);
+    const uint32_t k = ROW ? i : rank_in(a.obits, a.ooffs, device_key(a.g, x, y, z));
+    if (k >= (uint32_t)a.n) return;
+    a.perm[k] = (int)i;
+    a.coord[k] = (uint16_t)x;
+    a.coord[a.npad + k] = (uint16_t)y;
+    a.coord[2 * a.npad + k] = (uint16_t)z;
+}
+
+/* pull table, a thread per node */
+template <bool ROW>
+__global__ void k_nbr_from_flag(const TableArgs a)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= a.n) return;
+    const int x = a.coord[k], y = a.coord[a.npad + k], z = a.coord[2 * a.npad + k];
+    node_words<ROW>(a, x, y, z, ((size_t)z * a.g.ny + y) * a.g.nx + x, k);
 }
 
 /* --------------------------------------------------------- sphere pack */
@@ -167,52 +235,124 @@ __device__ __forceinline__ double min_image_d(double a, double c, int n)
     return d <= w ? d : w;
 }
 
-struct Sphere {
-    double cx, cy, cz, r;
-};
-
-/* one block per sphere: every cell of its bounding box that lies inside
- * takes the sphere's index if it is the first to cover it */
-__global__ void k_cover(const Sphere *sp, int base, int count, int nx, int ny,
-                        int nz, uint32_t *first)
+/* splitmix64 (Steele, Lea & Flood 2014), the same stream as plb_host.c: its
+ * k-th draw needs no draw before it */
+__device__ __forceinline__ double draw(uint64_t seed, uint64_t k)
 {
-    const int k = blockIdx.x;
-    if (k >= count) return;
-    const Sphere s = sp[k];
-    const double r2 = __dmul_rn(s.r, s.r);
-    int x0 = (int)floor(s.cx - s.r) - 1, x1 = (int)ceil(s.cx + s.r) + 1;
-    int y0 = (int)floor(s.cy - s.r) - 1, y1 = (int)ceil(s.cy + s.r) + 1;
-    int z0 = (int)floor(s.cz - s.r) - 1, z1 = (int)ceil(s.cz + s.r) + 1;
-    if (x1 - x0 + 1 > nx) x1 = x0 + nx - 1;
-    if (y1 - y0 + 1 > ny) y1 = y0 + ny - 1;
-    if (z1 - z0 + 1 > nz) z1 = z0 + nz - 1;
-    const int wx = x1 - x0 + 1, wy = y1 - y0 + 1, wz = z1 - z0 + 1;
-    const long long vol = (long long)wx * wy * wz;
-    const uint32_t idx = (uint32_t)(base + k);
-    for (long long t = threadIdx.x; t < vol; t += blockDim.x) {
-        const int X = x0 + (int)(t % wx);
-        const int Y = y0 + (int)((t / wx) % wy);
-        const int Z = z0 + (int)(t / ((long long)wx * wy));
+    uint64_t z = seed + (k + 1) * 0x9E3779B97F4A7C15ULL;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
+    z ^= z >> 31;
+    return __dmul_rn((double)(long long)(z >> 11), 0x1.0p-53);
+}
+
+/* cells along one axis of a sphere's bounding box that the tables hold */
+constexpr int kBox = 96;
+constexpr int kCoverThreads = 128;
+
+/* One block per sphere: every cell of its bounding box that lies inside
+ * takes the sphere's index if it is the first to cover it.  The squared
+ * distances along each axis are made once, in FP64 as the rule states, and
+ * kept in shared memory; a warp takes a row of cells along x and decides them
+ * in FP32 where the sum is clear of r^2 by more than FP32 can be off, in FP64
+ * where it is not.  In FP64 alone, nine operations a cell, the FP64 pipe
+ * bound the generator (200 x 192 x 210 cells, 18174 spheres: 2945 us, now
+ * 316). */
+__global__ void __launch_bounds__(kCoverThreads)
+k_cover(uint64_t seed, long long base, int nx, int ny, int nz, double rmin, double rmax,
+        uint32_t *first)
+{
+    __shared__ double d2[3][kBox];
+    __shared__ float f2[3][kBox]; /* (a conversion is an FP64-pipe operation) */
+    __shared__ int cell[3][kBox];
+    const long long s = base + blockIdx.x;
+    const uint32_t idx = (uint32_t)s;
+    const int n[3] = {nx, ny, nz};
+    const double c[3] = {__dmul_rn(draw(seed, 4 * s), (double)nx),
+                         __dmul_rn(draw(seed, 4 * s + 1), (double)ny),
+                         __dmul_rn(draw(seed, 4 * s + 2), (double)nz)};
+    const double r = __dadd_rn(rmin, __dmul_rn(__dsub_rn(rmax, rmin), draw(seed, 4 * s + 3)));
+    const double r2 = __dmul_rn(r, r);
+    int lo[3], w[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        lo[d] = (int)floor(c[d] - r) - 1;
+        int hi = (int)ceil(c[d] + r) + 1;
+        if (hi - lo[d] + 1 > n[d]) hi = lo[d] + n[d] - 1;
+        w[d] = hi - lo[d] + 1;
+    }
+    if (w[0] <= kBox && w[1] <= kBox && w[2] <= kBox) {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+            for (int t = threadIdx.x; t < w[d]; t += kCoverThreads) {
+                const int q = (((lo[d] + t) % n[d]) + n[d]) % n[d];
+                const double e = min_image_d((double)q, c[d], n[d]);
+                cell[d][t] = q;
+                d2[d][t] = __dmul_rn(e, e);
+                f2[d][t] = (float)d2[d][t];
+            }
+        __syncthreads();
+        /* FP32: each d2 and r2 rounded once, two adds: within 2^-22 */
+        const float in = (float)r2 * (1.f - 1e-6f), out = (float)r2 * (1.f + 1e-6f);
+        const int lane = threadIdx.x & 31;
+        const int rows = w[1] * w[2];
+        for (int row = threadIdx.x >> 5; row < rows; row += kCoverThreads / 32) {
+            const int iz = row / w[1], iy = row - iz * w[1];
+            const float dyz = f2[1][iy] + f2[2][iz];
+            if (dyz > out) continue;
+            uint32_t *const line = first + ((size_t)cell[2][iz] * ny + cell[1][iy]) * nx;
+            for (int ix = lane; ix < w[0]; ix += 32) {
+                const float e = f2[0][ix] + dyz;
+                if (e > out) continue;
+                if (e >= in &&
+                    !(__dadd_rn(__dadd_rn(d2[0][ix], d2[1][iy]), d2[2][iz]) <= r2))
+                    continue;
+                uint32_t *const p = line + cell[0][ix];
+                if (*(volatile uint32_t *)p > idx) atomicMin(p, idx);
+            }
+        }
+        return;
+    }
+    /* a box too wide for the tables: cell by cell */
+    const long long vol = (long long)w[0] * w[1] * w[2];
+    for (long long t = threadIdx.x; t < vol; t += kCoverThreads) {
+        const int X = lo[0] + (int)(t % w[0]);
+        const int Y = lo[1] + (int)((t / w[0]) % w[1]);
+        const int Z = lo[2] + (int)(t / ((long long)w[0] * w[1]));
         const int x = ((X % nx) + nx) % nx;
         const int y = ((Y % ny) + ny) % ny;
         const int z = ((Z % nz) + nz) % nz;
-        const double dx = min_image_d((double)x, s.cx, nx);
-        const double dy = min_image_d((double)y, s.cy, ny);
-        const double dz = min_image_d((double)z, s.cz, nz);
-        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                    __dmul_rn(dz, dz));
-        if (d2 <= r2) atomicMin(first + ((size_t)z * ny + y) * nx + x, idx);
+        const double dx = min_image_d((double)x, c[0], nx);
+        const double dy = min_image_d((double)y, c[1], ny);
+        const double dz = min_image_d((double)z, c[2], nz);
+        const double e = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
+                                   __dmul_rn(dz, dz));
+        if (e <= r2) atomicMin(first + ((size_t)z * ny + y) * nx + x, idx);
     }
 }
 
-/* hist[f - lo] += 1 for every cell first covered by sphere f in [lo, hi) */
+/* hist[f - lo] += 1 for every cell first covered by sphere f in [lo, hi);
+ * four cells a thread, runs of one sphere added at once */
 __global__ void k_first_hist(const uint32_t *first, size_t cells, uint32_t lo,
                              uint32_t hi, unsigned long long *hist)
 {
-    const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t c = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (c >= cells) return;
-    const uint32_t f = first[c];
-    if (f >= lo && f < hi) atomicAdd(hist + (f - lo), 1ull);
+    uint32_t f[4];
+    if (c + 4 <= cells) {
+        const uint4 v = *(const uint4 *)(first + c);
+        f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+    } else {
+        for (int k = 0; k < 4; k++) f[k] = c + k < cells ? first[c + k] : hi;
+    }
+    uint32_t run = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        run++;
+        if (k < 3 && f[k + 1] == f[k]) continue;
+        if (f[k] >= lo && f[k] < hi) atomicAdd(hist + (f[k] - lo), (unsigned long long)run);
+        run = 0;
+    }
 }
 
 __global__ void k_popc_words(const uint32_t *bits, uint32_t *cnt, size_t m)
@@ -224,9 +364,13 @@ __global__ void k_popc_words(const uint32_t *bits, uint32_t *cnt, size_t m)
 __global__ void k_flag_from_first(const uint32_t *first, size_t cells,
                                   uint32_t nsph, uint8_t *flag)
 {
-    const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cells) return;
-    flag[c] = first[c] < nsph ? 0 : 1;
+    const size_t c = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (c + 4 <= cells) {
+        const uint4 v = *(const uint4 *)(first + c);
+        *(uchar4 *)(flag + c) = make_uchar4(v.x >= nsph, v.y >= nsph, v.z >= nsph, v.w >= nsph);
+    } else {
+        for (size_t k = c; k < cells; k++) flag[k] = first[k] < nsph ? 0 : 1;
+    }
 }
 
 }  // namespace plb
@@ -246,16 +390,6 @@ static int ceil_log2i(int v)
     return b;
 }
 
-/* splitmix64 (Steele, Lea & Flood 2014), the same stream as plb_host.c */
-static uint64_t sm64(uint64_t *s)
-{
-    uint64_t z = (*s += 0x9E3779B97F4A7C15ULL);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-    return z ^ (z >> 31);
-}
-static double u01(uint64_t *s) { return (double)(sm64(s) >> 11) * 0x1.0p-53; }
-
 #define CKG(call)                                                             \
     do {                                                                      \
         cudaError_t e_ = (call);                                              \
@@ -267,6 +401,51 @@ static double u01(uint64_t *s) { return (double)(sm64(s) >> 11) * 0x1.0p-53; }
         }                                                                     \
     } while (0)
 
+/* Spheres drawn at a time: the expected count for the target porosity from
+ * the mean volume, and a third more. */
+static long long pack_chunk(size_t cells, double rmin, double rmax, double porosity)
+{
+    const double rm = 0.5 * (rmin + rmax);
+    const double v = 4.18879020478639 * rm * rm * rm;
+    const long long chunk =
+        (long long)(-log(porosity > 1e-6 ? porosity : 1e-6) * (double)cells / v * 1.3) + 64;
+    return chunk > 4000000 ? 4000000 : chunk;
+}
+
+static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+/* One device block for everything a geometry is made with. */
+int geom_alloc(GeomWork *w, int nx, int ny, int nz, int num_p)
+{
+    const size_t cells = (size_t)nx * ny * nz;
+    const size_t words = (cells + 31) / 32;
+    const size_t lines = up256(words * 4);
+    memset(w, 0, sizeof(*w));
+    const size_t tmp = up256(scan_tmp_bytes(words));
+    const size_t meta = up256(4 * ((size_t)num_p + 2));
+    if (plb_cuda_malloc(&w->block, up256(cells) + 3 * lines + tmp + meta) != cudaSuccess)
+        return PLB_ERR_NOMEM;
+    char *p = w->block;
+    w->flag = (uint8_t *)p;
+    p += up256(cells);
+    w->lexbits = (uint32_t *)p;
+    p += lines;
+    w->lexoffs = (uint32_t *)p;
+    p += lines;
+    w->cnt = (uint32_t *)p;
+    p += lines;
+    w->tmp = (uint32_t *)p;
+    p += tmp;
+    w->meta = (uint32_t *)p;
+    return PLB_OK;
+}
+
+void geom_free(GeomWork *w)
+{
+    cudaFree(w->block);
+    w->block = nullptr;
+}
+
 int sphere_pack_device(uint64_t seed, int nx, int ny, int nz, double rmin,
                        double rmax, double porosity, uint8_t *dflag,
                        int *num_spheres, double *porosity_out, cudaStream_t st)
@@ -275,43 +454,31 @@ int sphere_pack_device(uint64_t seed, int nx, int ny, int nz, double rmin,
     const double total = (double)cells;
     int rc = PLB_OK;
     uint32_t *first = nullptr;
-    Sphere *dsp = nullptr;
     unsigned long long *hist = nullptr;
-    Sphere *hsp = nullptr;
     unsigned long long *hh = nullptr;
-    uint64_t state = seed;
+    char *block = nullptr;
     long long made = 0, ns = -1;
     long long fluid = (long long)cells;
-    /* expected sphere count for the target porosity, from the mean volume */
-    const double rm = 0.5 * (rmin + rmax);
-    const double v = 4.18879020478639 * rm * rm * rm;
-    long long chunk = (long long)(-log(porosity > 1e-6 ? porosity : 1e-6) * total / v * 1.3) + 64;
-    if (chunk > 4000000) chunk = 4000000;
-    CKG(plb_cuda_malloc(&first, cells * 4));
+    const long long chunk = pack_chunk(cells, rmin, rmax, porosity);
+    const size_t hbytes = sizeof(unsigned long long) * (size_t)chunk;
+    CKG(plb_cuda_malloc(&block, up256(cells * 4) + hbytes));
+    first = (uint32_t *)block;
+    hist = (unsigned long long *)(block + up256(cells * 4));
     CKG(cudaMemsetAsync(first, 0xff, cells * 4, st));
-    CKG(plb_cuda_malloc(&dsp, sizeof(Sphere) * (size_t)chunk));
-    CKG(plb_cuda_malloc(&hist, sizeof(unsigned long long) * (size_t)chunk));
-    hsp = (Sphere *)malloc(sizeof(Sphere) * (size_t)chunk);
-    hh = (unsigned long long *)malloc(sizeof(unsigned long long) * (size_t)chunk);
-    if (!hsp || !hh) { rc = PLB_ERR_NOMEM; goto done; }
+    hh = (unsigned long long *)malloc(hbytes);
+    if (!hh) { rc = PLB_ERR_NOMEM; goto done; }
     if (!((double)fluid / total > porosity)) ns = 0;
     while (ns < 0) {
         if (made > 100000000LL) { rc = PLB_ERR_ARG; goto done; }
-        for (long long k = 0; k < chunk; k++) {
-            hsp[k].cx = u01(&state) * nx;
-            hsp[k].cy = u01(&state) * ny;
-            hsp[k].cz = u01(&state) * nz;
-            hsp[k].r = rmin + (rmax - rmin) * u01(&state);
-        }
-        CKG(cudaMemcpyAsync(dsp, hsp, sizeof(Sphere) * (size_t)chunk, cudaMemcpyHostToDevice, st));
-        k_cover<<<(unsigned)chunk, 256, 0, st>>>(dsp, (int)made, (int)chunk, nx, ny, nz, first);
+        k_cover<<<(unsigned)chunk, kCoverThreads, 0, st>>>(seed, made, nx, ny, nz, rmin, rmax,
+                                                          first);
         CKG(cudaGetLastError());
         /* cells first covered by each sphere of this chunk */
-        CKG(cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * (size_t)chunk, st));
-        k_first_hist<<<gsz(cells, 256), 256, 0, st>>>(first, cells, (uint32_t)made,
-                                                     (uint32_t)(made + chunk), hist);
+        CKG(cudaMemsetAsync(hist, 0, hbytes, st));
+        k_first_hist<<<gsz((cells + 3) / 4, 256), 256, 0, st>>>(first, cells, (uint32_t)made,
+                                                               (uint32_t)(made + chunk), hist);
         CKG(cudaGetLastError());
-        CKG(cudaMemcpyAsync(hh, hist, sizeof(unsigned long long) * (size_t)chunk, cudaMemcpyDeviceToHost, st));
+        CKG(cudaMemcpyAsync(hh, hist, hbytes, cudaMemcpyDeviceToHost, st));
         CKG(cudaStreamSynchronize(st));
         for (long long k = 0; k < chunk && ns < 0; k++) {
             fluid -= (long long)hh[k];
@@ -320,113 +487,116 @@ int sphere_pack_device(uint64_t seed, int nx, int ny, int nz, double rmin,
         made += chunk;
         if (ns < 0 && made + chunk > 0x7fffffffLL) { rc = PLB_ERR_ARG; goto done; }
     }
-    k_flag_from_first<<<gsz(cells, 256), 256, 0, st>>>(first, cells, (uint32_t)ns, dflag);
+    k_flag_from_first<<<gsz((cells + 3) / 4, 256), 256, 0, st>>>(first, cells, (uint32_t)ns,
+                                                                dflag);
     CKG(cudaGetLastError());
     CKG(cudaStreamSynchronize(st));
     if (num_spheres) *num_spheres = (int)ns;
     if (porosity_out) *porosity_out = (double)fluid / total;
 done:
     cudaStreamSynchronize(st);
-    cudaFree(first);
-    cudaFree(dsp);
-    cudaFree(hist);
-    free(hsp);
+    cudaFree(block);
     free(hh);
     return rc;
 }
 
-/* Lexicographic ranks of the fluid cells of a device flag grid.
- * lexbits/lexoffs: (cells+31)/32 words each.  *n receives the fluid count,
- * slab_start[num_p] the first node of every z slab. */
-int flag_rank(const uint8_t *dflag, int nx, int ny, int nz, int num_p,
-              uint32_t *lexbits, uint32_t *lexoffs, int *n, int *slab_start,
+/* Lexicographic ranks of the fluid cells of w's flag grid: bitmap and word
+ * offsets into w.  *n receives the fluid count, slab_start[num_p] the first
+ * node of every z slab. */
+int flag_rank(const GeomWork &w, int nx, int ny, int nz, int num_p, int *n, int *slab_start,
               cudaStream_t st)
 {
     const size_t cells = (size_t)nx * ny * nz;
     const size_t words = (cells + 31) / 32;
     int rc = PLB_OK;
-    unsigned *bad = nullptr;
-    uint32_t *cnt = nullptr;
-    unsigned hbad = 0;
-    CKG(plb_cuda_malloc(&bad, 4));
-    CKG(plb_cuda_malloc(&cnt, words * 4));
-    CKG(cudaMemsetAsync(bad, 0, 4, st));
-    k_flag_bits<<<gsz(words, 256), 256, 0, st>>>(dflag, cells, lexbits, cnt, words, bad);
+    uint32_t *h = (uint32_t *)malloc(4 * ((size_t)num_p + 2));
+    if (!h) return PLB_ERR_NOMEM;
+    CKG(cudaMemsetAsync(w.meta, 0, 8, st));
+    k_flag_bits<<<gsz(words, 256), 256, 0, st>>>(w.flag, cells, w.lexbits, w.cnt, words,
+                                                w.meta + 1);
     CKG(cudaGetLastError());
-    rc = scan_words(cnt, lexoffs, words, st);
+    rc = scan_words(w.cnt, w.lexoffs, words, w.tmp, st);
     if (rc != PLB_OK) goto done;
-    {
-        uint32_t last_off = 0, last_cnt = 0;
-        CKG(cudaMemcpyAsync(&last_off, lexoffs + words - 1, 4, cudaMemcpyDeviceToHost, st));
-        CKG(cudaMemcpyAsync(&last_cnt, cnt + words - 1, 4, cudaMemcpyDeviceToHost, st));
-        CKG(cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, st));
-        CKG(cudaStreamSynchronize(st));
-        if (hbad) { rc = PLB_ERR_ARG; goto done; }
-        const long long total = (long long)last_off + last_cnt;
-        if (total >= kMaxNodes) { rc = PLB_ERR_ARG; goto done; }
-        *n = (int)total;
-        /* slab starts: rank of the first cell of each slab (cell index is a
-         * multiple of 32 only when the plane is; count the remainder) */
-        const int slab = nz / num_p;
-        for (int p = 0; p < num_p; p++) {
-            const size_t c = (size_t)p * slab * nx * ny;
-            if (c >= cells) { slab_start[p] = *n; continue; }
-            uint32_t off = 0, word = 0;
-            CKG(cudaMemcpyAsync(&off, lexoffs + c / 32, 4, cudaMemcpyDeviceToHost, st));
-            CKG(cudaMemcpyAsync(&word, lexbits + c / 32, 4, cudaMemcpyDeviceToHost, st));
-            CKG(cudaStreamSynchronize(st));
-            slab_start[p] = (int)(off + __builtin_popcount(word & ((1u << (c & 31)) - 1u)));
-        }
+    k_rank_meta<<<gsz((size_t)num_p, 256), 256, 0, st>>>(w.lexbits, w.lexoffs, words, cells,
+                                                        (size_t)(nz / num_p) * nx * ny, num_p,
+                                                        w.meta);
+    CKG(cudaGetLastError());
+    CKG(cudaMemcpyAsync(h, w.meta, 4 * ((size_t)num_p + 2), cudaMemcpyDeviceToHost, st));
+    CKG(cudaStreamSynchronize(st));
+    if (h[1] || (long long)h[0] >= kMaxNodes) {
+        rc = PLB_ERR_ARG;
+        goto done;
     }
+    *n = (int)h[0];
+    for (int p = 0; p < num_p; p++) slab_start[p] = (int)h[2 + p];
 done:
-    cudaStreamSynchronize(st);
-    cudaFree(bad);
-    cudaFree(cnt);
+    free(h);
     return rc;
 }
 
 /* Morton (or reference) order, permutation, coordinates and pull table of
- * the fluid cells of a device flag grid, ranked by flag_rank. */
-int flag_tables(const uint8_t *dflag, int nx, int ny, int nz, int num_p,
-                int ordering, int remote_wins, int halfway, const uint32_t *lexbits,
-                const uint32_t *lexoffs, int n, long long npad, int *perm,
-                uint16_t *coord, uint32_t *nbr, uint32_t word_base,
-                uint32_t rest_word, cudaStream_t st)
+ * the fluid cells of w's flag grid, ranked by flag_rank; the node arrays
+ * perm and coord start at the domain's first node, nbr at the table's, whose
+ * node word_base is the domain's first.  Enqueued on st; the Morton order
+ * waits for it. */
+int flag_tables(const GeomWork &w, int nx, int ny, int nz, int num_p, int ordering,
+                int remote_wins, int halfway, int n, long long npad, int *perm, uint16_t *coord,
+                uint32_t *nbr, uint32_t word_base, uint32_t rest_word, cudaStream_t st)
 {
-    (void)dflag;
     const size_t cells = (size_t)nx * ny * nz;
-    Grid g{nx, ny, nz, ceil_log2i(nx), ceil_log2i(ny), ceil_log2i(nz),
-           ordering == PLB_ORDER_MORTON};
-    const int bits = g.morton ? g.bx + g.by + g.bz : 0;
-    if (bits > 40) return PLB_ERR_ARG;
-    const size_t space = g.morton ? ((size_t)1 << bits) : cells;
-    const size_t owords = (space + 31) / 32;
+    TableArgs a;
+    a.lexbits = w.lexbits;
+    a.lexoffs = w.lexoffs;
+    a.obits = a.ooffs = nullptr;
+    a.g = Grid{nx, ny, nz, ceil_log2i(nx), ceil_log2i(ny), ceil_log2i(nz),
+               ordering == PLB_ORDER_MORTON};
+    a.slab = nz / num_p;
+    a.remote_wins = remote_wins;
+    a.halfway = halfway;
+    a.n = n;
+    a.npad = npad;
+    a.word_base = word_base;
+    a.rest_word = rest_word;
+    a.perm = perm;
+    a.coord = coord;
+    a.nbr = nbr;
     int rc = PLB_OK;
-    uint32_t *obits = nullptr, *ooffs = nullptr, *ocnt = nullptr;
+    char *block = nullptr;
+    const int bits = a.g.morton ? a.g.bx + a.g.by + a.g.bz : 0;
+    if (bits > 40) return PLB_ERR_ARG;
     if (n == 0) return PLB_OK;
-    CKG(plb_cuda_malloc(&obits, owords * 4));
-    CKG(plb_cuda_malloc(&ooffs, owords * 4));
-    CKG(plb_cuda_malloc(&ocnt, owords * 4));
-    CKG(cudaMemsetAsync(obits, 0, owords * 4, st));
-    k_mark_order<<<gsz(cells, 256), 256, 0, st>>>(lexbits, g, cells, obits);
-    CKG(cudaGetLastError());
-    k_popc_words<<<gsz(owords, 256), 256, 0, st>>>(obits, ocnt, owords);
-    CKG(cudaGetLastError());
-    rc = scan_words(ocnt, ooffs, owords, st);
-    if (rc != PLB_OK) goto done;
-    k_assign_from_flag<<<gsz(cells, 256), 256, 0, st>>>(lexbits, lexoffs, obits, ooffs, g,
-                                                       cells, n, npad, perm, coord);
-    CKG(cudaGetLastError());
-    k_nbr_from_flag<<<gsz((size_t)n, 128), 128, 0, st>>>(lexbits, obits, ooffs, g, nz / num_p,
-                                                        remote_wins, halfway, n, npad,
-                                                        word_base, rest_word, coord, nbr);
-    CKG(cudaGetLastError());
-    CKG(cudaStreamSynchronize(st));
+    if (!a.g.morton) {
+        k_assign_from_flag<true><<<gsz(cells, 256), 256, 0, st>>>(a, cells);
+        CKG(cudaGetLastError());
+        k_nbr_from_flag<true><<<gsz((size_t)n, 128), 128, 0, st>>>(a);
+        CKG(cudaGetLastError());
+        return PLB_OK;
+    }
+    {
+        const size_t owords = (((size_t)1 << bits) + 31) / 32;
+        const size_t lines = up256(owords * 4);
+        CKG(plb_cuda_malloc(&block, 3 * lines + up256(scan_tmp_bytes(owords))));
+        uint32_t *obits = (uint32_t *)block, *ooffs = (uint32_t *)(block + lines),
+                 *ocnt = (uint32_t *)(block + 2 * lines);
+        CKG(cudaMemsetAsync(obits, 0, owords * 4, st));
+        k_mark_order<<<gsz(cells, 256), 256, 0, st>>>(w.lexbits, a.g, cells, obits);
+        CKG(cudaGetLastError());
+        k_popc_words<<<gsz(owords, 256), 256, 0, st>>>(obits, ocnt, owords);
+        CKG(cudaGetLastError());
+        rc = scan_words(ocnt, ooffs, owords, (uint32_t *)(block + 3 * lines), st);
+        if (rc != PLB_OK) goto done;
+        a.obits = obits;
+        a.ooffs = ooffs;
+        k_assign_from_flag<false><<<gsz(cells, 256), 256, 0, st>>>(a, cells);
+        CKG(cudaGetLastError());
+        k_nbr_from_flag<false><<<gsz((size_t)n, 128), 128, 0, st>>>(a);
+        CKG(cudaGetLastError());
+    }
 done:
-    cudaStreamSynchronize(st);
-    cudaFree(obits);
-    cudaFree(ooffs);
-    cudaFree(ocnt);
+    if (block) {
+        cudaStreamSynchronize(st);
+        cudaFree(block);
+    }
     return rc;
 }
 

@@ -173,21 +173,28 @@ struct BatchArgs {
  * present (plb_sim.cu). */
 void host_populate(void *p, size_t bytes);
 
-/* Exclusive scan of m uint32 counts into offs (device memory). */
-int scan_words(const uint32_t *cnt, uint32_t *offs, size_t m, cudaStream_t st);
+/* Exclusive scan of m uint32 counts into offs (device memory); tmp:
+ * scan_tmp_bytes(m) bytes. */
+size_t scan_tmp_bytes(size_t m);
+int scan_words(const uint32_t *cnt, uint32_t *offs, size_t m, uint32_t *tmp, cudaStream_t st);
 
-/* Device geometry (plb_geom.cu). */
+/* Device geometry (plb_geom.cu): the scratch of one build, in one block. */
+struct GeomWork {
+    char *block;
+    uint8_t *flag;               /* the flag grid */
+    uint32_t *lexbits, *lexoffs; /* fluid bitmap, rank of each word's first cell */
+    uint32_t *cnt, *tmp, *meta;
+};
+int geom_alloc(GeomWork *w, int nx, int ny, int nz, int num_p);
+void geom_free(GeomWork *w);
 int sphere_pack_device(uint64_t seed, int nx, int ny, int nz, double rmin,
                        double rmax, double porosity, uint8_t *dflag,
                        int *num_spheres, double *porosity_out, cudaStream_t st);
-int flag_rank(const uint8_t *dflag, int nx, int ny, int nz, int num_p,
-              uint32_t *lexbits, uint32_t *lexoffs, int *n, int *slab_start,
+int flag_rank(const GeomWork &w, int nx, int ny, int nz, int num_p, int *n, int *slab_start,
               cudaStream_t st);
-int flag_tables(const uint8_t *dflag, int nx, int ny, int nz, int num_p,
-                int ordering, int remote_wins, int halfway, const uint32_t *lexbits,
-                const uint32_t *lexoffs, int n, long long npad, int *perm,
-                uint16_t *coord, uint32_t *nbr, uint32_t word_base,
-                uint32_t rest_word, cudaStream_t st);
+int flag_tables(const GeomWork &w, int nx, int ny, int nz, int num_p, int ordering,
+                int remote_wins, int halfway, int n, long long npad, int *perm, uint16_t *coord,
+                uint32_t *nbr, uint32_t word_base, uint32_t rest_word, cudaStream_t st);
 
 /* Launch shape of a handle's steps. */
 struct StepLaunch {
