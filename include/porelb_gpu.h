@@ -118,7 +118,7 @@ typedef struct {
     int device;      /* CUDA device ordinal */
     int boundary;    /* PLB_BOUNDARY_REFERENCE (default) or PLB_BOUNDARY_HALFWAY */
     int kernel_variant; /* register budget of the step kernel: 0 (or 2) =
-                           default (PLB_FP64: 128 registers, 16 warps per SM;
+                           default (PLB_FP64: 96 registers, 20 warps per SM;
                            FP32/16-bit forms: 48 registers); 1 = 80 registers
                            (PLB_FP64) or unconstrained; 3 = 64 (PLB_FP64) or 40
                            registers.  Ignored by the other FP64 forms. */

@@ -263,13 +263,15 @@ FX_HD float rcp_rn(float x)
 }
 
 /*
- * One collision.  bits[19]: post-stream FP64 values (in), post-collision
- * FP64 values (out).  Returns kBad if the node must be recomputed in native
- * FP64, kDensity if the density guard trips.  mom receives rho*2^60, the
- * shifted momentum and 1/rho for the macro output.
+ * One collision.  bits[19]: post-stream FP64 values; store(j, bits) receives
+ * the post-collision values as they are made (holding all 19 to the end
+ * costs the registers of half the warps).  Returns kBad if the node must be
+ * recomputed in native FP64, kDensity if the density guard trips.  mom
+ * receives rho*2^60, the shifted momentum and 1/rho for the macro output.
  */
-FX_HD uint32_t collide(uint64_t (&bits)[19], const Consts &k, bool it_pos,
-                       Moments &mom)
+template <typename Store>
+FX_HD uint32_t collide(const uint64_t (&bits)[19], const Consts &k, bool it_pos,
+                       Moments &mom, const Store &store)
 {
     uint32_t chk = 0;
     int64_t D[19];
@@ -338,7 +340,7 @@ FX_HD uint32_t collide(uint64_t (&bits)[19], const Consts &k, bool it_pos,
     const int64_t W00 = Wv * 6 + k.wout[0];
 
     /* rest direction: e.J = 0 */
-    bits[0] = out_bits<0>(mul2(k.om1, split(D[0]), T00, split(-Ju15)) + W00, chk);
+    store(0, out_bits<0>(mul2(k.om1, split(D[0]), T00, split(-Ju15)) + W00, chk));
 #pragma unroll
     for (int J = 1; J < 19; J += 2) {
         const int K = J + 1;
@@ -367,14 +369,24 @@ FX_HD uint32_t collide(uint64_t (&bits)[19], const Consts &k, bool it_pos,
         const int64_t FnJ = mul2(k.om1, split(D[J]), TJ, split(qd + t3)) + WJ;
         const int64_t FnK = mul2(k.om1, split(D[K]), TK, split(qd - t3)) + WK;
         if (c == 1) {
-            bits[J] = out_bits<1>(FnJ, chk);
-            bits[K] = out_bits<1>(FnK, chk);
+            store(J, out_bits<1>(FnJ, chk));
+            store(K, out_bits<1>(FnK, chk));
         } else {
-            bits[J] = out_bits<2>(FnJ, chk);
-            bits[K] = out_bits<2>(FnK, chk);
+            store(J, out_bits<2>(FnJ, chk));
+            store(K, out_bits<2>(FnK, chk));
         }
     }
     return flags | ((chk >> 20) != 0u ? kBad : 0u);
+}
+
+/* the same, in place */
+FX_HD uint32_t collide(uint64_t (&bits)[19], const Consts &k, bool it_pos, Moments &mom)
+{
+    uint64_t out[19];
+    const uint32_t flags =
+        collide(bits, k, it_pos, mom, [&](int j, uint64_t v) { out[j] = v; });
+    for (int j = 0; j < 19; j++) bits[j] = out[j];
+    return flags;
 }
 
 }  // namespace fx

@@ -799,12 +799,12 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
     s->halo = p->halo;
     s->boundary = p->boundary;
     /* register budget of the step kernel (kernel_variant 1 and 3 are the
-     * alternatives; for FP64 the default 128-register kernel is the faster on
-     * GB300 - every tighter budget spills: 96 to 120 registers ran at 13.5 to
-     * 15.2 GLUPS at 256^3 against 16.2) */
+     * alternatives to the default) */
     s->variant = p->kernel_variant == 1 ? 1 : (p->kernel_variant == 3 ? 3 : 0);
     s->block = p->block_size > 0 ? p->block_size : step_block(p->precision, n);
     if (s->block > 256 || (s->block & 31)) s->block = 256;
+    /* the default FP64 kernel is built for CTAs of 128 threads at most */
+    if (p->precision == PLB_FP64 && s->variant == 0 && s->block > 128) s->variant = 4;
     /* prefetching the next wave into L2 pays for the issue-bound FP64 form
      * (+5% at 256^3 and 512^3) and costs the bandwidth-bound forms (FP32
      * -13%, FP16 deviations up to -11%) */

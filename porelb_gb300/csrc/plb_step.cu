@@ -374,20 +374,18 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float
 
 /* ----------------------------------------- FP64 on the integer pipes */
 
-template <bool MACRO>
-__device__ __forceinline__ Macro collide_fx(double (&f)[Q], const Coeffs &a,
-                                            bool &fallback)
+template <bool MACRO, typename Store>
+__device__ __forceinline__ Macro collide_fx(const double (&f)[Q], const Coeffs &a,
+                                            bool &fallback, const Store &store)
 {
     uint64_t b[Q];
 #pragma unroll
     for (int j = 0; j < Q; j++) b[j] = (uint64_t)__double_as_longlong(f[j]);
     fx::Moments mm;
-    const uint32_t fl = fx::collide(b, a.fxk, a.it > 0, mm);
+    const uint32_t fl = fx::collide(b, a.fxk, a.it > 0, mm, store);
     Macro m;
     fallback = (fl & fx::kBad) != 0;
     m.bad = (fl & fx::kDensity) != 0;
-#pragma unroll
-    for (int j = 0; j < Q; j++) f[j] = __longlong_as_double((long long)b[j]);
     if (MACRO) {
         uint32_t ignore = 0;
         m.rho = __longlong_as_double((long long)fx::to_bits(mm.R, ignore));
@@ -405,21 +403,31 @@ template <> struct StoreOf<PLB_FP32> { using T = float; };
 template <> struct StoreOf<PLB_FP16DEV> { using T = __half; };
 template <> struct StoreOf<PLB_BF16DEV> { using T = __nv_bfloat16; };
 
-/* Resident blocks of 256 threads per SM the register budget is set for,
- * by kernel variant (0 = default; 1 and 3 the alternatives the launch tuner
- * tries): fixed-point FP64 128 / 80 / 64 registers, the FP32 and 16-bit
- * forms 48 / unconstrained / 40 registers (48 is the faster on GB300: FP16
- * deviations 39.1 against 38.4 GLUPS at 512^3) or, with the words held before
- * the wait, 64 (at 48 they spill: FP16 at 92k nodes 2.94 against 2.75 us),
- * bit-exact FP64 80 (its
- * integer chains wait on themselves, so warps pay: 5.8 GLUPS at 256^3
- * against 4.9 with 108 registers and 16 warps per SM; 64 registers spill:
- * 5.7), FMA FP64 unconstrained. */
+/* Largest CTA (T) and resident CTAs of that size per SM (v) the register
+ * budget is set for, by kernel variant (0 = default; 1 and 3 the
+ * alternatives the launch tuner tries).
+ * Fixed-point FP64: 5 x 128 threads, 96 registers (322 us at 256^3, 1258 at
+ * 400^3; 128 registers 330 and 1368, 80 registers 333 and 1300: fewer warps
+ * wait longer, tighter budgets spill); 256-thread CTAs on request (V = 4) 128
+ * registers; the alternatives 80 and 64.
+ * FP32 and 16-bit forms: 48 registers (FP16 39.1 GLUPS at 512^3 against 38.4
+ * unconstrained) or, with the words held before the wait, 64 (at 48 they
+ * spill: FP16 at 92k nodes 2.94 against 2.75 us); the alternatives
+ * unconstrained and 40.
+ * Bit-exact FP64: 80 (its integer chains wait on themselves, so warps pay:
+ * 5.8 GLUPS at 256^3 against 4.9 with 108 registers and 16 warps per SM; 64
+ * registers spill: 5.7).  FMA FP64: unconstrained. */
 template <int PREC, int V, bool WF> struct MinBlocks {
     static constexpr bool dev = PREC == PLB_FP32 || PREC == PLB_FP16DEV || PREC == PLB_BF16DEV;
-    static constexpr int v = PREC == PLB_FP64 ? (V == 1 ? 3 : V == 3 ? 4 : 2)
+    static constexpr int T = PREC == PLB_FP64 && V == 0 ? 128 : 256;
+    static constexpr int v = PREC == PLB_FP64 ? (V == 1 ? 3 : V == 3 ? 4 : V == 4 ? 2 : 5)
                            : dev ? (V == 1 ? 1 : V == 3 ? 6 : WF ? 4 : 5)
                          : PREC == PLB_FP64_EXACT ? 3 : 1;
+    /* for the batch step's CTAs of BT threads */
+    static constexpr int batch(int BT)
+    {
+        return PREC == PLB_FP64 ? (BT == 128 ? 5 : 2) : v * (kBatchBlock / BT);
+    }
 };
 
 /* The bit-exact collision of node i outside plb_ex.h's common domain, from
@@ -492,16 +500,18 @@ __device__ __forceinline__ Macro collide_node(T (&raw)[Q], const T *fin, T *fout
     Macro m;
     if constexpr (PREC == PLB_FP64) {
         bool fallback;
-        m = collide_fx<MACRO>(raw, co, fallback);
+        m = collide_fx<MACRO>(raw, co, fallback, [&](int j, uint64_t v) {
+            __stcs(fout + (long long)j * np + i, __longlong_as_double((long long)v));
+        });
         if (fallback) {
             /* outside the fixed-point range: native FP64 from the streamed
-             * values, gathered again */
+             * values, gathered again, all 19 stored again */
             gather<T>(fin, nbr, np, i, raw);
             m = collide_fp64_fma(raw, co);
             flags |= 2u;
-        }
 #pragma unroll
-        for (int j = 0; j < Q; j++) __stcs(fout + (long long)j * np + i, raw[j]);
+            for (int j = 0; j < Q; j++) __stcs(fout + (long long)j * np + i, raw[j]);
+        }
     } else if constexpr (PREC == PLB_FP64_EXACT) {
         uint64_t b[Q];
 #pragma unroll
@@ -569,7 +579,8 @@ __device__ __forceinline__ void prefetch_block(const T *fin, const uint32_t *nbr
 }
 
 template <int PREC, bool MACRO, int VARIANT, bool WF>
-__global__ void __launch_bounds__(256, MinBlocks<PREC, VARIANT, WF>::v)
+__global__ void
+__launch_bounds__((MinBlocks<PREC, VARIANT, WF>::T), (MinBlocks<PREC, VARIANT, WF>::v))
 k_step(const StepArgs a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -640,7 +651,7 @@ k_step(const StepArgs a)
  * order their gathers share L2 lines (a fixed grid looping over the list
  * lost that and ran 23% slower in the FP64 form). */
 template <int PREC, bool MACRO, int BT, bool WF>
-__global__ void __launch_bounds__(BT, MinBlocks<PREC, 0, WF>::v * (kBatchBlock / BT))
+__global__ void __launch_bounds__(BT, (MinBlocks<PREC, 0, WF>::batch(BT)))
 k_batch_step(const BatchArgs a)
 {
     using T = typename StoreOf<PREC>::T;
@@ -806,6 +817,8 @@ static void (*step_variant(bool macros, bool wf, int variant))(StepArgs)
         if (variant == 1) return step_fn<PREC, 1>(macros, wf);
         if (variant == 3) return step_fn<PREC, 3>(macros, wf);
     }
+    if constexpr (PREC == PLB_FP64)
+        if (variant == 4) return step_fn<PREC, 4>(macros, wf);
     return step_fn<PREC, 0>(macros, wf);
 }
 
