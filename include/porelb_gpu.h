@@ -122,11 +122,10 @@ typedef struct {
                            FP32/16-bit forms: 48 registers); 1 = 80 registers
                            (PLB_FP64) or unconstrained; 3 = 64 (PLB_FP64) or 40
                            registers.  Ignored by the other FP64 forms. */
-    int l2_prefetch; /* L2 prefetch of the nodes of the blocks half a wave
-                        of resident blocks ahead:
-                        0 = the form's default (on for PLB_FP64, where it
-                        pays; off for the bandwidth-bound forms), 1 = on,
-                        -1 = off */
+    int l2_prefetch; /* L2 prefetch of the nodes of the blocks a fraction of
+                        a wave of resident blocks ahead: 0 = where it pays
+                        (PLB_FP64 and the 16-bit forms, for domains larger
+                        than the L2), 1 = on, -1 = off */
     int reserved[4];
 } plb_params;
 
@@ -302,9 +301,10 @@ typedef struct {
     int device;
     int cta_threads;       /* batch-step CTA: 128 or 256 threads (0: 128 for
                               PLB_FP64, 256 otherwise) */
-    int l2_prefetch;       /* L2 prefetch of the pool block half a wave
-                              ahead: 0 = default (on for PLB_FP64), 1 on,
-                              -1 off */
+    int l2_prefetch;       /* L2 prefetch of the pool block a fraction of a
+                              wave ahead: 0 = where it pays (PLB_FP64, FP32
+                              and 16-bit forms, for active samples larger
+                              than the L2 together), 1 on, -1 off */
     int ordering;          /* node order within each sample:
                               PLB_ORDER_MORTON (0, default),
                               PLB_ORDER_REFERENCE or PLB_ORDER_AUTO (chosen

@@ -258,7 +258,7 @@ struct plb_batch {
     bool in_flight = false;
     int cta = 256;     /* threads per CTA of the batch step */
     int ordering = PLB_ORDER_MORTON; /* node order of each sample's table */
-    int prefetch = 0;  /* L2 prefetch of the pool block half a wave ahead */
+    int prefetch = 0;  /* L2 prefetch: 1 on, -1 off, 0 where it pays */
     long long cap_blocks = 0, npad = 0, rest = 0;
     void *f[2] = {nullptr, nullptr};
     int cur = 0;
@@ -411,7 +411,7 @@ int plb_batch_create_ex(const plb_batch_params *bp, plb_batch **out)
     b->elem = elem_of(precision);
     b->cta = bp->cta_threads ? bp->cta_threads : batch_default_cta(precision);
     b->ordering = bp->ordering;
-    b->prefetch = bp->l2_prefetch > 0 || (bp->l2_prefetch == 0 && precision == PLB_FP64);
+    b->prefetch = bp->l2_prefetch;
     /* L2 groups on request: a budget in KiB, or -1 for 60% of the L2.  They
      * pay for pools of samples that fit in L2 (FP32 pools of 64^3 and 96^3
      * packs step 1.1-1.14x faster); on the batched workload, whose time goes
@@ -629,6 +629,13 @@ int plb_batch_add_packed(plb_batch *b, uint64_t seed, int nx, int ny, int nz,
     return rc;
 }
 
+/* L2 prefetch distance of a chain whose launches have `grid` CTAs. */
+static int chain_prefetch(const plb_batch *b, int grid)
+{
+    return prefetch_ctas(b->precision, (long long)grid * b->cta,
+                         batch_wave_blocks(b->precision, b->cta), true, b->prefetch);
+}
+
 /* A chain of K batch-step kernel nodes (the last writes the sums) from
  * buffer cur, over `grid` CTAs; with `grouped` the launches step the L2
  * group *gcur and a last node moves *gcur to the next group. */
@@ -641,8 +648,7 @@ static cudaError_t step_chain(plb_batch *b, bool grouped, int grid,
     a.nbr = b->nbr;
     a.npad = b->npad;
     a.blk_list = b->blist;
-    /* prefetch the pool block half a wave of CTAs ahead (FP64 by default) */
-    a.pf_blocks = b->prefetch ? (batch_wave_blocks(b->precision, b->cta) + 1) / 2 : 0;
+    a.pf_blocks = chain_prefetch(b, grid);
     const int h = B / b->cta;
     a.part_stride = h * b->cap_blocks;
     a.blk_sample = b->blk;
@@ -795,7 +801,9 @@ static int set_chain_grid(plb_batch *b, cudaGraphExec_t exec, std::vector<BatchA
     const void *fn = batch_step_kernel(b->precision, false, bt, grid);
     const void *fn_m = batch_step_kernel(b->precision, true, bt, grid);
     const int smem = batch_step_smem(b->precision, bt, grid);
+    const int pf = chain_prefetch(b, grid);
     for (int k = 0; k < b->K; k++) {
+        args[(size_t)k].pf_blocks = pf;
         void *kp[1] = {&args[(size_t)k]};
         cudaKernelNodeParams p;
         memset(&p, 0, sizeof(p));

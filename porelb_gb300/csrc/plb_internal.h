@@ -209,6 +209,8 @@ struct StepLaunch {
 int step_block(int precision, int n);
 /* fill in the rest of the shape for n nodes, given block and variant */
 void plan_step(int precision, int n, StepLaunch *l);
+/* L2 prefetch distance in CTAs of a plain or pool step launch (0: none) */
+int prefetch_ctas(int precision, long long nodes, int wave, bool pool, int want);
 /* launch one step of the given precision */
 cudaError_t launch_step(int precision, bool macros, const StepArgs &a, const StepLaunch &l,
                         cudaStream_t s);

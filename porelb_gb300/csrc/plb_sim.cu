@@ -34,7 +34,7 @@ struct plb_sim {
     int n, nx, ny, nz, num_p;
     long long npad;
     int precision, ordering, halo, block, boundary, variant;
-    int prefetch;     /* L2 prefetch on */
+    int prefetch;     /* L2 prefetch: 1 on, -1 off, 0 where it pays */
     StepLaunch shape; /* launch shape (planned at the first step) */
     int device;
     cudaStream_t stream;
@@ -805,10 +805,7 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
     if (s->block > 256 || (s->block & 31)) s->block = 256;
     /* the default FP64 kernel is built for CTAs of 128 threads at most */
     if (p->precision == PLB_FP64 && s->variant == 0 && s->block > 128) s->variant = 4;
-    /* prefetching the next wave into L2 pays for the issue-bound FP64 form
-     * (+5% at 256^3 and 512^3) and costs the bandwidth-bound forms (FP32
-     * -13%, FP16 deviations up to -11%) */
-    s->prefetch = p->l2_prefetch > 0 || (p->l2_prefetch == 0 && p->precision == PLB_FP64);
+    s->prefetch = p->l2_prefetch > 0 ? 1 : (p->l2_prefetch < 0 ? -1 : 0);
     s->device = p->device;
     s->elem = elem_size(p->precision);
     s->tau = p->tau;
@@ -1074,9 +1071,7 @@ int plb_step_async(plb_sim *s, int it_begin, int nsteps)
         plan_step(s->precision, s->n, &s->shape);
     }
     a.words_first = s->shape.words_first;
-    /* half a wave of resident blocks ahead (measured at 256^3 and 512^3:
-     * +0.7% against a whole wave, +7% against no prefetch) */
-    a.pf_blocks = s->prefetch ? (s->shape.wave + 1) / 2 : 0;
+    a.pf_blocks = prefetch_ctas(s->precision, s->n, s->shape.wave, false, s->prefetch);
     for (int k = 0; k < nsteps; k++) {
         a.fin = s->f[s->cur];
         a.fout = s->f[s->cur ^ 1];

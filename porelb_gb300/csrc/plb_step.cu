@@ -6,10 +6,10 @@
  * stream, stream_inner_nodes porelb.c:285-300), relaxes them (collision,
  * porelb.c:318-365) and writes its 19 post-collision values to the other
  * ping-pong buffer.  Distributions are SoA, f[j][npad], so the 19 stores and
- * the 18 neighbour-word loads of a warp are fully coalesced; the gathers hit
- * nodes that the Morton order keeps close in memory.  In the FP64 form each
- * CTA also asks L2 for the node range of the block half a wave of resident
- * blocks ahead (prefetch_block).
+ * the five neighbour-word loads of a warp are fully coalesced; the gathers hit
+ * nodes that the row or Morton order keeps close in memory.  On domains
+ * larger than the L2 each CTA also asks L2 for the node range of a block some
+ * way ahead (prefetch_block, prefetch_ctas).
  *
  * Forms:
  *   FP64_EXACT  the reference's operations in the reference's order with
@@ -842,13 +842,39 @@ static bool occupancy(const void *fn, int block, int *per, int *sms)
            cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, fn, block, 0) == cudaSuccess;
 }
 
+/* L2 prefetch distance in CTAs for a launch over `nodes` nodes, `wave` CTAs
+ * resident at once; want: 1 on, -1 off, 0 where it pays, which is once what a
+ * step moves outgrows the L2 (96^3 FP64, in L2: 22.3 us without, 23.2 with).
+ * Distances in 32nds of a wave, the fastest of 1 to 32:
+ *   plain step   FP64 8 (256^3: none 359 us, 8 318, 16 322), 16-bit 12 (FP16
+ *                none 141, 8 131, 12 129); FP32 loses (none 190, 8 193)
+ *   pool step    FP64 12 (16 x 96^3: none 334, 8 301, 12 294, 16 296), FP32 8
+ *                (none 162, 8 157, 24 163), 16-bit 16 (none 124, 8 114, 16 110) */
+int prefetch_ctas(int precision, long long nodes, int wave, bool pool, int want)
+{
+    const bool fp64 = precision == PLB_FP64;
+    const bool half = precision == PLB_FP16DEV || precision == PLB_BF16DEV;
+    const bool fp32 = precision == PLB_FP32;
+    if (want < 0) return 0;
+    if (want == 0) {
+        if (!fp64 && !half && !(fp32 && pool)) return 0;
+        int dev = 0, l2 = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+            return 0;
+        if (nodes * (2 * Q * (fp64 ? 8 : fp32 ? 4 : 2) + 72) <= l2) return 0;
+    }
+    const int part = half ? (pool ? 16 : 12) : fp64 && pool ? 12 : 8;
+    return (wave * part + 31) / 32;
+}
+
 template <int PREC>
 static void plan_prec(int n, StepLaunch *l)
 {
     int per = 0, sms = 0;
     const int grid = (n + l->block - 1) / l->block;
     /* blocks of the (non-macro) kernel resident on the whole device at once:
-     * the L2 prefetch distance */
+     * the unit of the L2 prefetch distance */
     l->wave = occupancy((const void *)step_variant<PREC>(false, false, l->variant), l->block,
                         &per, &sms) ? sms * per : 0;
     l->words_first = grid <= words_first_waves(PREC) * (long long)l->wave;

@@ -10,7 +10,7 @@ ordering and L2 prefetch.
   uses.
 * ``tune_pool`` (batched pool and server): for one storage form it builds a
   pool of synthetic sphere packs per candidate (batch-step CTAs of 128 or
-  256 threads, L2 prefetch of the pool block half a wave ahead on or off,
+  256 threads, L2 prefetch of the pool block a fraction of a wave ahead on or off,
   Morton or reference node order within each sample), times intervals of
   the batch step, and keeps the fastest.  Cached per
   form; every ``Batch`` created without an explicit launch takes the cached
