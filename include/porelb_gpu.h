@@ -124,8 +124,9 @@ typedef struct {
                            registers.  Ignored by the other FP64 forms. */
     int l2_prefetch; /* L2 prefetch of the nodes of the blocks a fraction of
                         a wave of resident blocks ahead: 0 = where it pays
-                        (PLB_FP64 and the 16-bit forms, for domains larger
-                        than the L2), 1 = on, -1 = off */
+                        (PLB_FP64 and the 16-bit forms, and PLB_FP32 in row
+                        order, for domains larger than the L2), 1 = on,
+                        -1 = off */
     int reserved[4];
 } plb_params;
 

@@ -188,16 +188,18 @@ __global__ void k_get_macro_sample(const double *macro, long long npad, long lon
 }
 
 /* a sample's node table moved into another pool: pull words re-based */
-__global__ void k_translate_words(const uint32_t *src, long long snp, long long sbase,
-                                  uint32_t srest, uint32_t *dst, long long dnp,
-                                  long long dbase, uint32_t drest, int n)
+__global__ void k_translate_words(const uint32_t *src, const uint8_t *sshorts, int plane,
+                                  long long srows, long long snp, long long sbase, uint32_t srest,
+                                  uint32_t *dst, long long drows, long long dnp, long long dbase,
+                                  uint32_t drest, int n)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     uint32_t words[Q - 1];
 #pragma unroll
     for (int j = 1; j < Q; j++) {
-        const uint32_t w = src[word_at(j, sbase + k, snp)];
+        const uint32_t w =
+            (uint32_t)word_of(src, sshorts, j, sbase + k, srows, snp, plane, (int)srest);
         uint32_t o;
         if (w == srest) o = drest;
         else if ((long long)(uint32_t)(w - (uint32_t)sbase) < (long long)n)
@@ -205,7 +207,7 @@ __global__ void k_translate_words(const uint32_t *src, long long snp, long long 
         else o = bounce_word(j, dbase + k, dnp);
         words[j - 1] = o;
     }
-    store_words(dst, dnp, dbase + k, words);
+    store_words(dst, dbase + k, drows, words);
 }
 
 /* a sample's stored deviations moved into another storage form: g =
@@ -263,6 +265,7 @@ struct plb_batch {
     void *f[2] = {nullptr, nullptr};
     int cur = 0;
     uint32_t *nbr = nullptr;
+    uint8_t *shorts = nullptr; /* pool blocks with short words (forms that read them) */
     int *perm = nullptr;
     uint16_t *coord = nullptr;
     double *macro = nullptr;
@@ -337,6 +340,7 @@ static void batch_free(plb_batch *b)
     cudaFree(b->f[0]);
     cudaFree(b->f[1]);
     cudaFree(b->nbr);
+    cudaFree(b->shorts);
     cudaFree(b->perm);
     cudaFree(b->coord);
     cudaFree(b->macro);
@@ -440,7 +444,10 @@ int plb_batch_create_ex(const plb_batch_params *bp, plb_batch **out)
     const size_t np = (size_t)b->npad;
     al(&b->f[0], b->elem * Q * np);
     al(&b->f[1], b->elem * Q * np);
-    al(&b->nbr, 4 * 18 * np);
+    al(&b->nbr, 4 * word_count(precision, b->npad));
+    /* L2 groups step inside the L2, where short words only cost */
+    if (short_words_pay(precision, b->rest) && !b->group_bytes)
+        al(&b->shorts, (size_t)b->npad / kWordNodes);
     al(&b->perm, 4 * np);
     al(&b->coord, 2 * 3 * np);
     if (keep_macros) al(&b->macro, 8 * 4 * np);
@@ -457,6 +464,8 @@ int plb_batch_create_ex(const plb_batch_params *bp, plb_batch **out)
     if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_ssum, 8 * 3 * (size_t)max_samples);
     if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_serr, 4 * (size_t)max_samples);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->blk, 0xff, 4 * (size_t)b->cap_blocks, b->st);
+    if (e == cudaSuccess && b->shorts)
+        e = cudaMemsetAsync(b->shorts, 0, (size_t)b->npad / kWordNodes, b->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->sactive, 0, 4 * (size_t)max_samples, b->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->serr, 0, 4 * (size_t)max_samples, b->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->t_dev, 0, 4, b->st);
@@ -540,7 +549,12 @@ static int add_dflag(plb_batch *b, const GeomWork &w, int nx, int ny, int nz,
                               ? plb_auto_ordering(n, nz, (int)b->elem, b->device)
                               : b->ordering;
         rc = flag_tables(w, nx, ny, nz, 1, order, 0, 0, n, b->npad, b->perm + base, b->coord + base,
-                         b->nbr, (uint32_t)base, (uint32_t)b->rest, b->adm);
+                         b->nbr, word_rows(b->precision, b->npad), (uint32_t)base, (uint32_t)b->rest,
+                         b->adm);
+        if (rc == PLB_OK && b->shorts &&
+            shorten_words(b->nbr, b->shorts, base, n, n / nz, (int)b->rest, true, nullptr,
+                          b->adm) != cudaSuccess)
+            rc = PLB_ERR_CUDA;
         if (rc != PLB_OK) free_range(b, blk0, nblk);
     }
     if (rc != PLB_OK) return rc;
@@ -573,6 +587,7 @@ static int add_dflag(plb_batch *b, const GeomWork &w, int nx, int ny, int nz,
     make_coeffs(sp->tau, sp->force_x, h.scale, &d.co);
     d.base = blk0 * B;
     d.n = n;
+    d.plane = n / nz;
     /* a sample admitted while an interval runs starts after it */
     d.start = (int)(b->t + (b->in_flight ? b->K : 0));
     h.start = d.start;
@@ -633,7 +648,8 @@ int plb_batch_add_packed(plb_batch *b, uint64_t seed, int nx, int ny, int nz,
 static int chain_prefetch(const plb_batch *b, int grid)
 {
     return prefetch_ctas(b->precision, (long long)grid * b->cta,
-                         batch_wave_blocks(b->precision, b->cta), true, b->prefetch);
+                         batch_wave_blocks(b->precision, b->cta), true, b->shorts != nullptr,
+                         b->prefetch);
 }
 
 /* A chain of K batch-step kernel nodes (the last writes the sums) from
@@ -646,6 +662,8 @@ static cudaError_t step_chain(plb_batch *b, bool grouped, int grid,
     BatchArgs a;
     memset(&a, 0, sizeof(a));
     a.nbr = b->nbr;
+    a.shorts = b->shorts;
+    a.rest = (int)b->rest;
     a.npad = b->npad;
     a.blk_list = b->blist;
     a.pf_blocks = chain_prefetch(b, grid);
@@ -662,9 +680,9 @@ static cudaError_t step_chain(plb_batch *b, bool grouped, int grid,
         a.grp_cur = b->gcur;
     }
     const int bt = b->cta;
-    const void *fn = batch_step_kernel(b->precision, false, bt, grid);
-    const void *fn_m = batch_step_kernel(b->precision, true, bt, grid);
-    const int smem = batch_step_smem(b->precision, bt, grid);
+    const void *fn = batch_step_kernel(b->precision, false, bt, grid, b->shorts);
+    const void *fn_m = batch_step_kernel(b->precision, true, bt, grid, b->shorts);
+    const int smem = batch_step_smem(b->precision, bt, grid, b->shorts);
     args.assign((size_t)b->K, a);
     nodes.assign((size_t)b->K, nullptr);
     cudaGraph_t g = nullptr;
@@ -798,9 +816,9 @@ static int set_chain_grid(plb_batch *b, cudaGraphExec_t exec, std::vector<BatchA
                           std::vector<cudaGraphNode_t> &nodes, int grid)
 {
     const int bt = b->cta;
-    const void *fn = batch_step_kernel(b->precision, false, bt, grid);
-    const void *fn_m = batch_step_kernel(b->precision, true, bt, grid);
-    const int smem = batch_step_smem(b->precision, bt, grid);
+    const void *fn = batch_step_kernel(b->precision, false, bt, grid, b->shorts);
+    const void *fn_m = batch_step_kernel(b->precision, true, bt, grid, b->shorts);
+    const int smem = batch_step_smem(b->precision, bt, grid, b->shorts);
     const int pf = chain_prefetch(b, grid);
     for (int k = 0; k < b->K; k++) {
         args[(size_t)k].pf_blocks = pf;
@@ -1116,15 +1134,19 @@ int plb_batch_transfer(plb_batch *src, int id, plb_batch *dst, int *new_id)
             e = cudaMemcpyAsync(dst->coord + r * dst->npad + db, src->coord + r * src->npad + sb,
                                 2 * (size_t)n, cudaMemcpyDeviceToDevice, dst->adm);
         if (e == cudaSuccess) {
-            k_translate_words<<<gb(n, B), B, 0, dst->adm>>>(src->nbr, src->npad, sb,
-                                                           (uint32_t)src->rest, dst->nbr,
-                                                           dst->npad, db, (uint32_t)dst->rest, n);
+            k_translate_words<<<gb(n, B), B, 0, dst->adm>>>(
+                src->nbr, src->shorts, hs.dev.plane, word_rows(src->precision, src->npad),
+                src->npad, sb, (uint32_t)src->rest, dst->nbr,
+                word_rows(dst->precision, dst->npad), dst->npad, db, (uint32_t)dst->rest, n);
+            if (dst->shorts)
+                e = shorten_words(dst->nbr, dst->shorts, db, n, n / hs.nz, (int)dst->rest, true,
+                                  nullptr, dst->adm);
             switch (src->precision) {
             case PLB_FP32: convert_to<float>(src, hs, dst, db, scale); break;
             case PLB_FP16DEV: convert_to<__half>(src, hs, dst, db, scale); break;
             default: convert_to<__nv_bfloat16>(src, hs, dst, db, scale); break;
             }
-            e = cudaGetLastError();
+            if (e == cudaSuccess) e = cudaGetLastError();
         }
     }
     if (e != cudaSuccess) {
@@ -1152,6 +1174,7 @@ int plb_batch_transfer(plb_batch *src, int id, plb_batch *dst, int *new_id)
     make_coeffs(h.tau, h.force, h.scale, &d.co);
     d.base = db;
     d.n = n;
+    d.plane = n / h.nz;
     d.start = (int)h.start;
     BCK(cudaMemcpyAsync(dst->sdev + sid, &d, sizeof(d), cudaMemcpyHostToDevice, dst->adm));
     BCK(cudaMemsetAsync(dst->serr + sid, 0, 4, dst->adm));

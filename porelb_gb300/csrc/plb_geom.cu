@@ -127,7 +127,7 @@ struct TableArgs {
     const uint32_t *obits, *ooffs;     /* device order (Morton) */
     Grid g;
     int slab, remote_wins, halfway, n;
-    long long npad;
+    long long npad, rows;
     uint32_t word_base, rest_word;
     int *perm;
     uint16_t *coord;
@@ -177,7 +177,7 @@ __device__ __forceinline__ void node_words(const TableArgs &a, int x, int y, int
                          ? bounce_word(j, (long long)a.word_base + k, a.npad)
                          : a.rest_word;
     }
-    store_words(a.nbr, a.npad, (long long)a.word_base + k, words);
+    store_words(a.nbr, (long long)a.word_base + k, a.rows, words);
 }
 
 /* x, y, z of a cell */
@@ -222,6 +222,51 @@ __global__ void k_nbr_from_flag(const TableArgs a)
     if (k >= a.n) return;
     const int x = a.coord[k], y = a.coord[a.npad + k], z = a.coord[2 * a.npad + k];
     node_words<ROW>(a, x, y, z, ((size_t)z * a.g.ny + y) * a.g.nx + x, k);
+}
+
+/* One CTA per block of 256 nodes; see shorten_words. */
+__global__ void __launch_bounds__(kWordNodes)
+k_shorten_words(uint32_t *nbr, uint8_t *shorts, long long lo, int n, int plane, int rest,
+                int rewrite, int *count)
+{
+    const long long blk = (lo >> 8) + blockIdx.x;
+    const long long i = blk * kWordNodes + threadIdx.x;
+    bool fits = true;
+    uint32_t q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (i < lo + n) {
+#pragma unroll
+        for (int j = 1; j < Q; j++) {
+            const int s = (int)nbr[word_at(j, i, 0)];
+            long long d = kShortBounce;
+            if (s == rest) {
+                d = kShortRest;
+            } else if (s >= lo && s < lo + n) {
+                d = s - i - (long long)dz_planes(j) * plane + kShortBias;
+                fits = fits && d >= 0 && d < kShortBounce;
+            }
+            q[(j - 1) >> 1] |= ((uint32_t)d & 0xffffu) << ((j & 1) ? 0 : 16);
+        }
+    }
+    /* every word of the block has been read when the first is rewritten */
+    const bool all = __syncthreads_and(fits);
+    if (threadIdx.x == 0) {
+        shorts[blk] = (uint8_t)all;
+        if (all && count) atomicAdd(count, 1);
+    }
+    if (!all || !rewrite) return;
+    uint32_t *p = nbr + blk * kWordBlock;
+    ((uint4 *)p)[threadIdx.x] = make_uint4(q[0], q[1], q[2], q[3]);
+    ((uint4 *)p)[256 + threadIdx.x] = make_uint4(q[4], q[5], q[6], q[7]);
+    p[2048 + threadIdx.x] = q[8];
+}
+
+cudaError_t shorten_words(uint32_t *nbr, uint8_t *shorts, long long lo, int n, int plane,
+                          int rest, bool rewrite, int *count, cudaStream_t st)
+{
+    if (n <= 0) return cudaSuccess;
+    k_shorten_words<<<(unsigned)((n + kWordNodes - 1) / kWordNodes), kWordNodes, 0, st>>>(
+        nbr, shorts, lo, n, plane, rest, rewrite, count);
+    return cudaGetLastError();
 }
 
 /* --------------------------------------------------------- sphere pack */
@@ -541,7 +586,8 @@ done:
  * waits for it. */
 int flag_tables(const GeomWork &w, int nx, int ny, int nz, int num_p, int ordering,
                 int remote_wins, int halfway, int n, long long npad, int *perm, uint16_t *coord,
-                uint32_t *nbr, uint32_t word_base, uint32_t rest_word, cudaStream_t st)
+                uint32_t *nbr, long long rows, uint32_t word_base, uint32_t rest_word,
+                cudaStream_t st)
 {
     const size_t cells = (size_t)nx * ny * nz;
     TableArgs a;
@@ -555,6 +601,7 @@ int flag_tables(const GeomWork &w, int nx, int ny, int nz, int num_p, int orderi
     a.halfway = halfway;
     a.n = n;
     a.npad = npad;
+    a.rows = rows;
     a.word_base = word_base;
     a.rest_word = rest_word;
     a.perm = perm;

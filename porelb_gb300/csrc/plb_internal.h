@@ -63,32 +63,106 @@ __host__ __device__ constexpr int wclass(int j)
  * 2 * npad < 2^31, hence kMaxNodes. */
 constexpr long long kMaxNodes = (1LL << 30) - 512;
 
-/* The 18 words of a node lie in five rows, four of four words and one of
- * two, so that a thread reads them with four 16-byte loads and one 8-byte
- * load: where word j of node i is. */
-__host__ __device__ constexpr long long word_at(int j, long long i, long long npad)
-{
-    return j <= 16 ? (long long)((j - 1) & ~3) * npad + 4 * i + ((j - 1) & 3)
-                   : 16 * npad + 2 * i + (j - 17);
-}
-
-#if defined(__CUDACC__)
-/* store the words w[j - 1] of node i */
-__device__ __forceinline__ void store_words(uint32_t *nbr, long long npad, long long i,
-                                            const uint32_t (&w)[18])
-{
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-        *(uint4 *)(nbr + word_at(4 * q + 1, i, npad)) =
-            make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-    *(uint2 *)(nbr + word_at(17, i, npad)) = make_uint2(w[16], w[17]);
-}
-#endif
-
 __host__ __device__ inline uint32_t bounce_word(int j, long long i, long long npad)
 {
     return (uint32_t)(i + (long long)(opp(j) - j) * npad);
 }
+
+/* The 18 words of a node lie in five rows, four of four words a node and one
+ * of two, so that a thread reads them with four 16-byte loads and one 8-byte
+ * load.  Where word j of node i is: in rows of `rows` nodes or, rows 0, with
+ * the words of 256 nodes together, which is what short words need (the forms
+ * without them lose 0.5-2% by it: FP64 96^3 22.5 against 22.1 us, FP16 7.0
+ * against 6.8). */
+constexpr int kWordNodes = 256;
+constexpr int kWordBlock = 18 * kWordNodes;
+__host__ __device__ constexpr long long word_in_rows(int j, long long i, long long rows)
+{
+    return j <= 16 ? (long long)((j - 1) & ~3) * rows + 4 * i + ((j - 1) & 3)
+                   : 16 * rows + 2 * i + (j - 17);
+}
+__host__ __device__ constexpr long long word_in_block(int j, long long i)
+{
+    return (i >> 8) * kWordBlock + (j <= 16 ? ((j - 1) >> 2) * 1024 + 4 * (i & 255) + ((j - 1) & 3)
+                                            : 4096 + 2 * (i & 255) + (j - 17));
+}
+__host__ __device__ constexpr long long word_at(int j, long long i, long long rows)
+{
+    return rows ? word_in_rows(j, i, rows) : word_in_block(j, i);
+}
+
+/* Short words.  In row order the sources of direction j lie close to i +
+ * dz_planes(j) * plane, with plane the domain's mean nodes per z-plane.  A
+ * block of 256 nodes whose sources all lie within 16 bits of that keeps its
+ * words as 16-bit distances instead, in the first half of its place: two rows
+ * of eight and one of two.  Two more values mean the node's own reversed
+ * value and the rest slot.  All blocks but those at the periodic wraps fit
+ * (98-99% at 128^3 to 400^3), and a step of the FP32 form, which streams at
+ * the copy rate, reads 36 bytes a node less (256^3: 190 -> 163 us, 36 GLUPS). */
+constexpr int kShortBias = 32767; /* distance d is kept as d + kShortBias */
+constexpr uint32_t kShortBounce = 0xfffe;
+constexpr uint32_t kShortRest = 0xffff;
+__host__ __device__ constexpr int dz_planes(int j) { return -ez(j); }
+/* the forms whose steps can read short words (see short_words_pay) */
+__host__ __device__ constexpr bool short_form(int precision) { return precision == PLB_FP32; }
+/* word_at()'s rows for a form, and the words allocated for npad nodes */
+__host__ __device__ constexpr long long word_rows(int precision, long long npad)
+{
+    return short_form(precision) ? 0 : npad;
+}
+inline size_t word_count(int precision, long long npad)
+{
+    if (!short_form(precision)) return 18 * (size_t)npad;
+    return (size_t)((npad + kWordNodes - 1) / kWordNodes) * kWordBlock;
+}
+
+#if defined(__CUDACC__)
+/* store the words w[j - 1] of node i */
+__device__ __forceinline__ void store_words(uint32_t *nbr, long long i, long long rows,
+                                            const uint32_t (&w)[18])
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        *(uint4 *)(nbr + word_at(4 * q + 1, i, rows)) =
+            make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+    *(uint2 *)(nbr + word_at(17, i, rows)) = make_uint2(w[16], w[17]);
+}
+
+/* the short words of node i (two to an entry) */
+__device__ __forceinline__ void load_short(const uint32_t *nbr, long long i, uint32_t (&q)[9])
+{
+    const uint32_t *p = nbr + (i >> 8) * kWordBlock;
+    const int t = (int)(i & 255);
+    const uint4 a = __ldg((const uint4 *)p + t), b = __ldg((const uint4 *)p + 256 + t);
+    q[0] = a.x; q[1] = a.y; q[2] = a.z; q[3] = a.w;
+    q[4] = b.x; q[5] = b.y; q[6] = b.z; q[7] = b.w;
+    q[8] = __ldg(p + 2048 + t);
+}
+
+/* the pull word of direction j that node i's short words stand for */
+__device__ __forceinline__ int short_word(const uint32_t (&q)[9], int j, int i, long long npad,
+                                          int plane, int rest)
+{
+    const uint32_t pair = q[(j - 1) >> 1];
+    const bool high = !(j & 1);
+    const uint32_t w = high ? pair >> 16 : pair & 0xffffu;
+    int o = (i + dz_planes(j) * plane - kShortBias) + (int)w;
+    if (high ? pair >= (kShortBounce << 16) : w >= kShortBounce) o = i + (opp(j) - j) * (int)npad;
+    if (high ? pair >= (kShortRest << 16) : w >= kShortRest) o = rest;
+    return o;
+}
+
+/* the pull word of direction j of node i, whichever way its block is kept */
+__device__ __forceinline__ int word_of(const uint32_t *nbr, const uint8_t *shorts, int j,
+                                       long long i, long long rows, long long npad, int plane,
+                                       int rest)
+{
+    if (!shorts || !shorts[i >> 8]) return (int)nbr[word_at(j, i, rows)];
+    uint32_t q[9];
+    load_short(nbr, i, q);
+    return short_word(q, j, (int)i, npad, plane, rest);
+}
+#endif
 
 /* Per-solve collision coefficients (host-computed from tau and F). */
 struct Coeffs {
@@ -109,6 +183,9 @@ struct StepArgs {
     const void *fin;
     void *fout;
     const uint32_t *nbr;  /* word_at() */
+    const uint8_t *shorts; /* blocks of 256 nodes with short words; may be NULL */
+    int plane;             /* mean nodes per z-plane (short words) */
+    int rest;              /* the rest slot */
     const int *perm;      /* new -> reference index (density guard report) */
     long long npad;
     int n;
@@ -119,9 +196,13 @@ struct StepArgs {
     unsigned long long *err; /* min over (it << 32 | reference index) */
     unsigned int *flags;     /* bit 0: FP16 scale overflow, bit 1: fallback */
     int pf_blocks;           /* L2 prefetch distance in blocks (0 = none) */
-    int words_first;         /* load the neighbour words before waiting for the
-                                step before (see words_first_waves) */
+    int words_first;         /* the FP64 form's kernels, built for both, load
+                                the words before the wait */
 };
+
+/* How a step kernel reads its words: whole ones after the wait for the step
+ * before, or before it (see words_first_waves); short ones (before it). */
+enum WordMode { kWordsLate, kWordsFirst, kWordsShort };
 
 /* Waves of resident CTAs up to which a step loads its words before it waits
  * for the step before; above it, the gathers go out as their words arrive.
@@ -143,12 +224,15 @@ struct SampleDev {
     long long base; /* first node of the sample in the pool */
     int n;          /* fluid nodes */
     int start;      /* batch step at which the sample started */
+    int plane;      /* mean nodes per z-plane (short words) */
 };
 
 struct BatchArgs {
     const void *fin;
     void *fout;
     const uint32_t *nbr;
+    const uint8_t *shorts;     /* pool blocks with short words; may be NULL */
+    int rest;                  /* the rest slot */
     long long npad;
     const int *blk_list;       /* pool blocks this launch covers (one CTA each,
                                   two for 128-thread CTAs) */
@@ -194,14 +278,24 @@ int flag_rank(const GeomWork &w, int nx, int ny, int nz, int num_p, int *n, int 
               cudaStream_t st);
 int flag_tables(const GeomWork &w, int nx, int ny, int nz, int num_p, int ordering,
                 int remote_wins, int halfway, int n, long long npad, int *perm, uint16_t *coord,
-                uint32_t *nbr, uint32_t word_base, uint32_t rest_word, cudaStream_t st);
+                uint32_t *nbr, long long rows, uint32_t word_base, uint32_t rest_word,
+                cudaStream_t st);
+
+/* Short words for the blocks of nodes lo .. lo + n - 1 (lo a multiple of 256)
+ * whose sources are near: flags the blocks in shorts, counts them in *count
+ * (device memory, may be NULL) and, with `rewrite`, rewrites their words. */
+cudaError_t shorten_words(uint32_t *nbr, uint8_t *shorts, long long lo, int n, int plane,
+                          int rest, bool rewrite, int *count, cudaStream_t st);
+
+/* whether `nodes` nodes step faster with short words */
+bool short_words_pay(int precision, long long nodes);
 
 /* Launch shape of a handle's steps. */
 struct StepLaunch {
     int block;       /* threads per CTA */
     int variant;     /* register budget (plb_params.kernel_variant) */
     int wave;        /* CTAs resident on the device at once (0: not planned) */
-    int words_first; /* as StepArgs */
+    int words;       /* WordMode */
     int smem;        /* shared memory that spreads the grid over the SMs */
 };
 
@@ -210,7 +304,7 @@ int step_block(int precision, int n);
 /* fill in the rest of the shape for n nodes, given block and variant */
 void plan_step(int precision, int n, StepLaunch *l);
 /* L2 prefetch distance in CTAs of a plain or pool step launch (0: none) */
-int prefetch_ctas(int precision, long long nodes, int wave, bool pool, int want);
+int prefetch_ctas(int precision, long long nodes, int wave, bool pool, bool shorts, int want);
 /* launch one step of the given precision */
 cudaError_t launch_step(int precision, bool macros, const StepArgs &a, const StepLaunch &l,
                         cudaStream_t s);
@@ -225,9 +319,9 @@ int batch_default_cta(int precision);
  * CTAs each) for a launch of `grid` CTAs, for a graph kernel node; NULL for
  * another size. */
 constexpr int kBatchBlock = 256;
-const void *batch_step_kernel(int precision, bool macros, int cta, int grid);
+const void *batch_step_kernel(int precision, bool macros, int cta, int grid, bool shorts);
 /* its shared memory (see spread_smem) */
-int batch_step_smem(int precision, int cta, int grid);
+int batch_step_smem(int precision, int cta, int grid, bool shorts);
 
 /* Fill the coefficients from tau, F and the storage scale. */
 void make_coeffs(double tau, double force, float scale, Coeffs *c);

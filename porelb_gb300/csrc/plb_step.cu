@@ -80,18 +80,27 @@ __device__ __forceinline__ void pdl_wait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+/* word_at() for the form that stores T (FP32 alone has short words) */
+template <typename T>
+__device__ __forceinline__ long long word_place(int j, long long i, long long np)
+{
+    if constexpr (sizeof(T) == 4) return word_in_block(j, i);
+    return word_in_rows(j, i, np);
+}
+
+template <typename T>
 __device__ __forceinline__ void load_words(const uint32_t *nbr, long long np, long long i,
                                            int (&w)[Q - 1])
 {
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        const int4 v = __ldg((const int4 *)(nbr + word_at(4 * q + 1, i, np)));
+        const int4 v = __ldg((const int4 *)(nbr + word_place<T>(4 * q + 1, i, np)));
         w[4 * q] = v.x;
         w[4 * q + 1] = v.y;
         w[4 * q + 2] = v.z;
         w[4 * q + 3] = v.w;
     }
-    const int2 v = __ldg((const int2 *)(nbr + word_at(17, i, np)));
+    const int2 v = __ldg((const int2 *)(nbr + word_place<T>(17, i, np)));
     w[16] = v.x;
     w[17] = v.y;
 }
@@ -111,7 +120,7 @@ __device__ __forceinline__ void gather(const T *fin, const uint32_t *nbr,
                                        long long np, long long i, T (&f)[Q])
 {
     int w[Q - 1];
-    load_words(nbr, np, i, w);
+    load_words<T>(nbr, np, i, w);
     gather_words<T>(fin, np, i, w, f);
 }
 
@@ -124,13 +133,24 @@ __device__ __forceinline__ void stream_node(const void *fin, const uint32_t *nbr
 {
     if constexpr (WF) {
         int w[Q - 1];
-        if (valid) load_words(nbr, np, i, w);
+        if (valid) load_words<T>(nbr, np, i, w);
         pdl_wait();
         if (valid) gather_words<T>((const T *)fin, np, i, w, f);
     } else {
         pdl_wait();
         if (valid) gather<T>((const T *)fin, nbr, np, i, f);
     }
+}
+
+/* the streamed values of node i from its short words q */
+template <typename T>
+__device__ __forceinline__ void gather_short(const T *fin, const uint32_t (&q)[9], long long np,
+                                             long long i, int plane, int rest, T (&f)[Q])
+{
+    f[0] = fin[i];
+#pragma unroll
+    for (int j = 1; j < Q; j++)
+        f[j] = fin[(long long)j * np + short_word(q, j, (int)i, np, plane, rest)];
 }
 
 /* ------------------------------------------------- FP64, reference order */
@@ -417,11 +437,11 @@ template <> struct StoreOf<PLB_BF16DEV> { using T = __nv_bfloat16; };
  * Bit-exact FP64: 80 (its integer chains wait on themselves, so warps pay:
  * 5.8 GLUPS at 256^3 against 4.9 with 108 registers and 16 warps per SM; 64
  * registers spill: 5.7).  FMA FP64: unconstrained. */
-template <int PREC, int V, bool WF> struct MinBlocks {
+template <int PREC, int V, int W> struct MinBlocks {
     static constexpr bool dev = PREC == PLB_FP32 || PREC == PLB_FP16DEV || PREC == PLB_BF16DEV;
     static constexpr int T = PREC == PLB_FP64 && V == 0 ? 128 : 256;
     static constexpr int v = PREC == PLB_FP64 ? (V == 1 ? 3 : V == 3 ? 4 : V == 4 ? 2 : 5)
-                           : dev ? (V == 1 ? 1 : V == 3 ? 6 : WF ? 4 : 5)
+                           : dev ? (V == 1 ? 1 : V == 3 ? 6 : W == kWordsFirst ? 4 : 5)
                          : PREC == PLB_FP64_EXACT ? 3 : 1;
     /* for the batch step's CTAs of BT threads */
     static constexpr int batch(int BT)
@@ -557,36 +577,53 @@ __device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes)
 
 /* Thread 0 of a block asks L2 for the node range of block b (a block that
  * starts some time after this one, pf_blocks blocks later in launch order):
- * its five rows of neighbour words and its 19 rows of distributions.  In
+ * its rows of neighbour words and its 19 rows of distributions.  In
  * Morton order most gathers of that block read inside the ranges of the
- * blocks launched near it, so its loads then wait for L2 instead of DRAM.  Rows are npad elements (a
- * multiple of 64) and the block size is a multiple of 32, so every range
- * starts 64-byte aligned and spans a multiple of 64 bytes inside its row. */
+ * blocks launched near it, so its loads then wait for L2 instead of DRAM.
+ * Rows are npad elements (a multiple of 64) and the block size is a multiple
+ * of 32, so every range starts 64-byte aligned and spans a multiple of 64
+ * bytes inside its row or its word block. */
 template <typename T>
 __device__ __forceinline__ void prefetch_block(const T *fin, const uint32_t *nbr,
-                                               long long np, long long n, long long b,
-                                               int bs)
+                                               const uint8_t *shorts, long long np, long long n,
+                                               long long b, int bs)
 {
     const long long i0 = b * bs;
     if (i0 >= n) return;
     const long long cnt = np - i0 < bs ? np - i0 : bs;
     const unsigned fb = (unsigned)(cnt * (long long)sizeof(T));
+    /* one range or, where the words of 256 nodes lie together, one for each
+     * such block that this one touches */
+    for (long long k = i0; k < i0 + cnt;) {
+        long long end = i0 + cnt;
+        if (sizeof(T) == 4 && (k | 255) + 1 < end) end = (k | 255) + 1;
+        const unsigned m = (unsigned)(end - k);
+        if (shorts && shorts[k >> 8]) {
+            const uint32_t *p = nbr + (k >> 8) * kWordBlock;
+            prefetch_l2(p + 4 * (k & 255), m * 16);
+            prefetch_l2(p + 1024 + 4 * (k & 255), m * 16);
+            prefetch_l2(p + 2048 + (k & 255), m * 4);
+        } else {
 #pragma unroll 1
-    for (int j = 1; j < 17; j += 4) prefetch_l2(nbr + word_at(j, i0, np), (unsigned)(cnt * 16));
-    prefetch_l2(nbr + word_at(17, i0, np), (unsigned)(cnt * 8));
+            for (int j = 1; j < 17; j += 4) prefetch_l2(nbr + word_place<T>(j, k, np), m * 16);
+            prefetch_l2(nbr + word_place<T>(17, k, np), m * 8);
+        }
+        k = end;
+    }
 #pragma unroll 1
     for (int j = 0; j < Q; j++) prefetch_l2(fin + (long long)j * np + i0, fb);
 }
 
-template <int PREC, bool MACRO, int VARIANT, bool WF>
+template <int PREC, bool MACRO, int VARIANT, int W>
 __global__ void
-__launch_bounds__((MinBlocks<PREC, VARIANT, WF>::T), (MinBlocks<PREC, VARIANT, WF>::v))
+__launch_bounds__((MinBlocks<PREC, VARIANT, W>::T), (MinBlocks<PREC, VARIANT, W>::v))
 k_step(const StepArgs a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.pf_blocks > 0 && threadIdx.x == 0)
         prefetch_block<typename StoreOf<PREC>::T>((const typename StoreOf<PREC>::T *)a.fin,
-                                                  a.nbr, a.npad, a.n,
+                                                  a.nbr, W == kWordsShort ? a.shorts : nullptr,
+                                                  a.npad, a.n,
                                                   (long long)blockIdx.x + a.pf_blocks,
                                                   blockDim.x);
     using T = typename StoreOf<PREC>::T;
@@ -599,8 +636,23 @@ k_step(const StepArgs a)
          * lose to a branch */
         if (a.words_first) stream_node<T, true>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
         else stream_node<T, false>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
+    } else if constexpr (W == kWordsShort) {
+        /* the short words are asked for before it is known whether the block
+         * has them: a block that has not (1 in 60) reads 36 bytes a node
+         * for nothing, the others wait for one load less */
+        uint32_t q[9];
+        bool is_short = false;
+        if (i < a.n) {
+            load_short(a.nbr, i, q);
+            is_short = __ldg(a.shorts + (i >> 8)) != 0;
+        }
+        pdl_wait();
+        if (i < a.n) {
+            if (is_short) gather_short<T>((const T *)a.fin, q, a.npad, i, a.plane, a.n, raw);
+            else gather<T>((const T *)a.fin, a.nbr, a.npad, i, raw);
+        }
     } else {
-        stream_node<T, WF>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
+        stream_node<T, W == kWordsFirst>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
     }
     double sum_u = 0.0, sum_r = 0.0;
     if (i < a.n) {
@@ -650,8 +702,8 @@ k_step(const StepArgs a)
  * that run at the same time work on neighbouring pool blocks, so in Morton
  * order their gathers share L2 lines (a fixed grid looping over the list
  * lost that and ran 23% slower in the FP64 form). */
-template <int PREC, bool MACRO, int BT, bool WF>
-__global__ void __launch_bounds__(BT, (MinBlocks<PREC, 0, WF>::batch(BT)))
+template <int PREC, bool MACRO, int BT, int W>
+__global__ void __launch_bounds__(BT, (MinBlocks<PREC, 0, W>::batch(BT)))
 k_batch_step(const BatchArgs a)
 {
     using T = typename StoreOf<PREC>::T;
@@ -675,7 +727,8 @@ k_batch_step(const BatchArgs a)
     /* L2 prefetch of the part of a pool block the CTA pf_blocks later steps */
     if (a.pf_blocks > 0 && threadIdx.x == 0 && (int)blockIdx.x + a.pf_blocks < ncta) {
         const unsigned c = blockIdx.x + a.pf_blocks;
-        prefetch_block<T>((const T *)a.fin, a.nbr, a.npad, a.npad,
+        prefetch_block<T>((const T *)a.fin, a.nbr, W == kWordsShort ? a.shorts : nullptr,
+                          a.npad, a.npad,
                           (long long)list[c / H] * H + c % H, BT);
     }
     double sum_u = 0.0, sum_r = 0.0;
@@ -685,7 +738,18 @@ k_batch_step(const BatchArgs a)
      * writes them, so they are read before the wait (see k_step) */
     T raw[Q];
     pdl_launch_next();
-    stream_node<T, WF>(a.fin, a.nbr, a.npad, i, valid, raw);
+    if (W == kWordsShort && a.shorts[pb]) {
+        uint32_t q[9];
+        int plane = 0;
+        if (valid) {
+            load_short(a.nbr, i, q);
+            plane = a.samples[s].plane;
+        }
+        pdl_wait();
+        if (valid) gather_short<T>((const T *)a.fin, q, a.npad, i, plane, a.rest, raw);
+    } else {
+        stream_node<T, W == kWordsFirst>(a.fin, a.nbr, a.npad, i, valid, raw);
+    }
     if (valid) {
         {
             /* the sample's coefficients straight from global memory (the
@@ -801,25 +865,29 @@ static int spread_smem(Fn fn, Fn fn_macros, int grid, int block)
 }
 
 template <int PREC, int V>
-static void (*step_fn(bool macros, bool wf))(StepArgs)
+static void (*step_fn(bool macros, int words))(StepArgs)
 {
+    if constexpr (short_form(PREC))
+        if (words == kWordsShort)
+            return macros ? k_step<PREC, true, V, kWordsShort> : k_step<PREC, false, V, kWordsShort>;
     if constexpr (PREC != PLB_FP64)
-        if (wf) return macros ? k_step<PREC, true, V, true> : k_step<PREC, false, V, true>;
-    return macros ? k_step<PREC, true, V, false> : k_step<PREC, false, V, false>;
+        if (words == kWordsFirst)
+            return macros ? k_step<PREC, true, V, kWordsFirst> : k_step<PREC, false, V, kWordsFirst>;
+    return macros ? k_step<PREC, true, V, kWordsLate> : k_step<PREC, false, V, kWordsLate>;
 }
 
 /* the tighter register budgets are built for the tuned forms only */
 template <int PREC>
-static void (*step_variant(bool macros, bool wf, int variant))(StepArgs)
+static void (*step_variant(bool macros, int words, int variant))(StepArgs)
 {
     if constexpr (PREC == PLB_FP64 || PREC == PLB_FP32 || PREC == PLB_FP16DEV ||
                   PREC == PLB_BF16DEV) {
-        if (variant == 1) return step_fn<PREC, 1>(macros, wf);
-        if (variant == 3) return step_fn<PREC, 3>(macros, wf);
+        if (variant == 1) return step_fn<PREC, 1>(macros, words);
+        if (variant == 3) return step_fn<PREC, 3>(macros, words);
     }
     if constexpr (PREC == PLB_FP64)
-        if (variant == 4) return step_fn<PREC, 4>(macros, wf);
-    return step_fn<PREC, 0>(macros, wf);
+        if (variant == 4) return step_fn<PREC, 4>(macros, words);
+    return step_fn<PREC, 0>(macros, words);
 }
 
 template <int PREC>
@@ -828,7 +896,7 @@ static cudaError_t launch_prec(bool macros, const StepArgs &a, const StepLaunch 
 {
     const int grid = (a.n + l.block - 1) / l.block;
     if (grid == 0) return cudaSuccess;
-    return launch_pdl(step_variant<PREC>(macros, a.words_first != 0, l.variant), grid, l.block,
+    return launch_pdl(step_variant<PREC>(macros, l.words, l.variant), grid, l.block,
                       l.smem, a, s);
 }
 
@@ -842,30 +910,56 @@ static bool occupancy(const void *fn, int block, int *per, int *sms)
            cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, fn, block, 0) == cudaSuccess;
 }
 
+/* L2 bytes of the current device, 0 if unknown */
+static int l2_bytes()
+{
+    int dev = 0, l2 = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+                   cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess
+               ? l2 : 0;
+}
+
 /* L2 prefetch distance in CTAs for a launch over `nodes` nodes, `wave` CTAs
  * resident at once; want: 1 on, -1 off, 0 where it pays, which is once what a
  * step moves outgrows the L2 (96^3 FP64, in L2: 22.3 us without, 23.2 with).
  * Distances in 32nds of a wave, the fastest of 1 to 32:
  *   plain step   FP64 8 (256^3: none 359 us, 8 318, 16 322), 16-bit 12 (FP16
- *                none 141, 8 131, 12 129); FP32 loses (none 190, 8 193)
- *   pool step    FP64 12 (16 x 96^3: none 334, 8 301, 12 294, 16 296), FP32 8
- *                (none 162, 8 157, 24 163), 16-bit 16 (none 124, 8 114, 16 110) */
-int prefetch_ctas(int precision, long long nodes, int wave, bool pool, int want)
+ *                none 141, 8 131, 12 129), FP32 6 with short words (none 166,
+ *                4 163, 6 163, 16 166); with wide ones FP32 loses (none 190,
+ *                8 193)
+ *   pool step    FP64 12 (16 x 96^3: none 334, 8 301, 12 294, 16 296), FP32 16
+ *                with short words (none 141, 8 142, 16 139) and 8 without (none
+ *                162, 8 157, 24 163), 16-bit 16 (none 124, 8 114, 16 110) */
+int prefetch_ctas(int precision, long long nodes, int wave, bool pool, bool shorts, int want)
 {
     const bool fp64 = precision == PLB_FP64;
     const bool half = precision == PLB_FP16DEV || precision == PLB_BF16DEV;
     const bool fp32 = precision == PLB_FP32;
     if (want < 0) return 0;
     if (want == 0) {
-        if (!fp64 && !half && !(fp32 && pool)) return 0;
-        int dev = 0, l2 = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
+        if (!fp64 && !half && !(fp32 && (pool || shorts))) return 0;
+        const int l2 = l2_bytes();
+        if (l2 <= 0 || nodes * (2 * Q * (fp64 ? 8 : fp32 ? 4 : 2) + (shorts ? 36 : 72)) <= l2)
             return 0;
-        if (nodes * (2 * Q * (fp64 ? 8 : fp32 ? 4 : 2) + 72) <= l2) return 0;
     }
-    const int part = half ? (pool ? 16 : 12) : fp64 && pool ? 12 : 8;
+    const int part = half  ? (pool ? 16 : 12)
+                     : fp64 ? (pool ? 12 : 8)
+                     : pool ? (shorts ? 16 : 8)
+                            : (shorts ? 6 : 8);
     return (wave * part + 31) / 32;
+}
+
+/* Short words cost a step about 100 instructions a node and save it 36 of 224
+ * bytes of DRAM traffic, so they are for node sets that outgrow the L2
+ * (FP32, wide then short: 96^3 6.7 and 8.1 us, 108^3 12.5 and 11.3, 128^3
+ * 25.3 and 22.0, 256^3 190 and 166, 400^3 715 and 627).  The line lies
+ * at two thirds of it (393k nodes; 108^3 has 441k).  The 16-bit forms are
+ * not bound by DRAM (256^3 FP16 with short words 137 us, with wide 129) and
+ * neither are the FP64 ones (327 and 318). */
+bool short_words_pay(int precision, long long nodes)
+{
+    return short_form(precision) && l2_bytes() > 0 &&
+           nodes * (2 * Q * 4 + 72) > l2_bytes() / 3 * 2;
 }
 
 template <int PREC>
@@ -875,11 +969,11 @@ static void plan_prec(int n, StepLaunch *l)
     const int grid = (n + l->block - 1) / l->block;
     /* blocks of the (non-macro) kernel resident on the whole device at once:
      * the unit of the L2 prefetch distance */
-    l->wave = occupancy((const void *)step_variant<PREC>(false, false, l->variant), l->block,
+    l->wave = occupancy((const void *)step_variant<PREC>(false, kWordsLate, l->variant), l->block,
                         &per, &sms) ? sms * per : 0;
-    l->words_first = grid <= words_first_waves(PREC) * (long long)l->wave;
-    l->smem = spread_smem(step_variant<PREC>(false, l->words_first != 0, l->variant),
-                          step_variant<PREC>(true, l->words_first != 0, l->variant), grid,
+    l->words = grid <= words_first_waves(PREC) * (long long)l->wave ? kWordsFirst : kWordsLate;
+    l->smem = spread_smem(step_variant<PREC>(false, l->words, l->variant),
+                          step_variant<PREC>(true, l->words, l->variant), grid,
                           l->block);
 }
 
@@ -939,7 +1033,7 @@ template <int PREC, int BT>
 static int batch_wave_bt()
 {
     int per = 0, sms = 0;
-    return occupancy((const void *)k_batch_step<PREC, false, BT, true>, BT, &per, &sms) ? sms * per
+    return occupancy((const void *)k_batch_step<PREC, false, BT, kWordsFirst>, BT, &per, &sms) ? sms * per
                                                                                       : 0;
 }
 
@@ -963,15 +1057,20 @@ int batch_wave_blocks(int precision, int cta)
 }
 
 template <int PREC, int BT>
-static const void *batch_fn(bool macros, bool wf)
+static const void *batch_fn(bool macros, int words)
 {
-    if constexpr (MinBlocks<PREC, 0, true>::dev) {
-        if (!wf)
-            return macros ? (const void *)k_batch_step<PREC, true, BT, false>
-                          : (const void *)k_batch_step<PREC, false, BT, false>;
+    if constexpr (short_form(PREC)) {
+        if (words == kWordsShort)
+            return macros ? (const void *)k_batch_step<PREC, true, BT, kWordsShort>
+                          : (const void *)k_batch_step<PREC, false, BT, kWordsShort>;
     }
-    return macros ? (const void *)k_batch_step<PREC, true, BT, true>
-                  : (const void *)k_batch_step<PREC, false, BT, true>;
+    if constexpr (MinBlocks<PREC, 0, kWordsFirst>::dev) {
+        if (words == kWordsLate)
+            return macros ? (const void *)k_batch_step<PREC, true, BT, kWordsLate>
+                          : (const void *)k_batch_step<PREC, false, BT, kWordsLate>;
+    }
+    return macros ? (const void *)k_batch_step<PREC, true, BT, kWordsFirst>
+                  : (const void *)k_batch_step<PREC, false, BT, kWordsFirst>;
 }
 
 /* The pool's words come first in every launch of the FP64 forms (0.1M to 6M
@@ -979,29 +1078,32 @@ static const void *batch_fn(bool macros, bool wf)
  * the same number of waves as a plain step's (FP32 92k nodes 3.6 against 3.9
  * us, 5M nodes 171 against 162). */
 template <int PREC>
-static const void *batch_fn_cta(bool macros, int cta, int grid)
+static const void *batch_fn_cta(bool macros, int cta, int grid, bool shorts)
 {
-    const bool wf = grid <= (long long)words_first_waves(PREC) * batch_wave_prec<PREC>(cta);
-    return cta == 128 ? batch_fn<PREC, 128>(macros, wf) : batch_fn<PREC, kBatchBlock>(macros, wf);
+    const int words = shorts ? kWordsShort
+                      : grid <= (long long)words_first_waves(PREC) * batch_wave_prec<PREC>(cta)
+                          ? kWordsFirst : kWordsLate;
+    return cta == 128 ? batch_fn<PREC, 128>(macros, words)
+                      : batch_fn<PREC, kBatchBlock>(macros, words);
 }
 
-int batch_step_smem(int precision, int cta, int grid)
+int batch_step_smem(int precision, int cta, int grid, bool shorts)
 {
-    const void *fn = batch_step_kernel(precision, false, cta, grid);
-    const void *fn_m = batch_step_kernel(precision, true, cta, grid);
+    const void *fn = batch_step_kernel(precision, false, cta, grid, shorts);
+    const void *fn_m = batch_step_kernel(precision, true, cta, grid, shorts);
     return fn && fn_m ? spread_smem(fn, fn_m, grid, cta) : 0;
 }
 
-const void *batch_step_kernel(int precision, bool macros, int cta, int grid)
+const void *batch_step_kernel(int precision, bool macros, int cta, int grid, bool shorts)
 {
     if (cta != 128 && cta != kBatchBlock) return nullptr;
     switch (precision) {
-    case PLB_FP64_EXACT: return batch_fn_cta<PLB_FP64_EXACT>(macros, cta, grid);
-    case PLB_FP64: return batch_fn_cta<PLB_FP64>(macros, cta, grid);
-    case PLB_FP64_FMA: return batch_fn_cta<PLB_FP64_FMA>(macros, cta, grid);
-    case PLB_FP32: return batch_fn_cta<PLB_FP32>(macros, cta, grid);
-    case PLB_FP16DEV: return batch_fn_cta<PLB_FP16DEV>(macros, cta, grid);
-    case PLB_BF16DEV: return batch_fn_cta<PLB_BF16DEV>(macros, cta, grid);
+    case PLB_FP64_EXACT: return batch_fn_cta<PLB_FP64_EXACT>(macros, cta, grid, shorts);
+    case PLB_FP64: return batch_fn_cta<PLB_FP64>(macros, cta, grid, shorts);
+    case PLB_FP64_FMA: return batch_fn_cta<PLB_FP64_FMA>(macros, cta, grid, shorts);
+    case PLB_FP32: return batch_fn_cta<PLB_FP32>(macros, cta, grid, shorts);
+    case PLB_FP16DEV: return batch_fn_cta<PLB_FP16DEV>(macros, cta, grid, shorts);
+    case PLB_BF16DEV: return batch_fn_cta<PLB_BF16DEV>(macros, cta, grid, shorts);
     default: return nullptr;
     }
 }
