@@ -79,17 +79,22 @@ struct plb_sim {
 
 int plb_auto_ordering(long long n, int nz, int elem_bytes, int device)
 {
-    /* bytes a step moves per node: 19 values in and out, 18 words, perm */
-    const double bpn = 2.0 * 19 * elem_bytes + 72 + 4;
+    /* bytes a step moves per node: 19 values in and out, 18 words (short ones
+     * in the form that has them), perm */
+    const bool shorts = elem_bytes == 4;
+    const double bpn = 2.0 * 19 * elem_bytes + (shorts ? 36 : 72) + 4;
     int l2 = 0;
     if (nz <= 0 || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) != cudaSuccess ||
         l2 <= 0)
         return PLB_ORDER_MORTON;
     const double plane = bpn * (double)n / nz;
     /* measured: row order wins up to about 63 MB of such planes on a 126 MB
-     * L2 (512^3 FP32) and loses from 105 MB (512^3 FP64, whose L2 prefetch
-     * also takes room) */
-    return 3.0 * plane <= 0.6 * (double)l2 ? PLB_ORDER_REFERENCE : PLB_ORDER_MORTON;
+     * L2 (512^3 FP16) and loses from 105 MB (512^3 FP64, whose L2 prefetch
+     * also takes room).  FP32 keeps short words in row order only: 35.9
+     * against 30.3 GLUPS at 30 MB (512^3, porosity 0.2), 34.9 / 30.5 at 121
+     * (1024^3), 32.1 / 30.3 at 211 (1024^3, porosity 0.35), the largest
+     * measured */
+    return 3.0 * plane <= (shorts ? 1.75 : 0.6) * (double)l2 ? PLB_ORDER_REFERENCE : PLB_ORDER_MORTON;
 }
 
 /* ------------------------------------------------------ allocation */

@@ -14,7 +14,7 @@ requests that arrive while others run overlaps on the device with theirs.
 Storage forms:
 * one pool in FP32 (default), FP64, FP16 or BF16 deviations;
 * ``"fp16dev"`` with ``handoff_tol``: requests start in a pool of scaled
-  FP16 deviations (148 B per lattice update against FP32's 224) and, once
+  FP16 deviations (148 B per lattice update against FP32's 188 to 224) and, once
   the relative change of <u_x> over an interval falls below handoff_tol,
   move with their state and history into an FP32 pool, where the
   steady-state test finishes at the request's own tolerance.  FP16

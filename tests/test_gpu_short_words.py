@@ -44,6 +44,14 @@ def test_row_and_morton_order_agree(dims, solid, boundary):
     assert np.allclose(got[0][3], got[1][3], rtol=1e-12, atol=0)
 
 
+def test_large_domains_keep_row_order():
+    """FP32 row order is for planes up to 1.75 times the L2 (short words),
+    measured up to 1024^3 at porosity 0.35."""
+    assert P.auto_ordering(214748328, 1024, "fp32") == "reference"
+    assert P.auto_ordering(375808416, 1024, "fp32") == "reference"
+    assert P.auto_ordering(900000000, 1024, "fp32") == "morton"
+
+
 def test_records_of_many_ranks():
     """Tables built from node records of several ranks, against Morton order."""
     dims = (120, 90, 80)
