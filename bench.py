@@ -35,6 +35,15 @@ FALLBACK_HBM = 6800.0
 BYTES_PER_NODE = {"fp64_exact": 376, "fp64": 376, "fp64_fma": 376, "fp32": 224,
                   "fp16dev": 148, "bf16dev": 148}
 
+
+def bytes_per_node(prec, num_node, order):
+    """The FP32 form keeps 16-bit words (36 bytes instead of 72) in row order
+    on domains that outgrow the L2."""
+    if prec == "fp32" and order == "reference" and num_node > 400000:
+        return 188
+    return BYTES_PER_NODE[prec]
+
+
 # DRAM bytes (read + write) of one step-kernel launch come from one-pass ncu
 # captures summarised in profiles/*.md, each with a line
 #   traffic-record: workload=W form=F num_node=N order=O bytes=B source=D
@@ -403,7 +412,7 @@ def run_gpu(args, rank, world, local):
     peak, peak_kind = hbm_peak()
     order = P.auto_ordering(N, dims[2], prec, local)
     traffic, traffic_src = recorded_traffic(args.workload, prec, N, order)
-    bpn = BYTES_PER_NODE[prec]
+    bpn = bytes_per_node(prec, N, order)
     achieved = bpn * N / (ms_step * 1e-3) / 1e9
     line = {
         "metric": METRIC, "value": round(value, 3), "unit": "MLUPS",
@@ -802,7 +811,8 @@ def run_precision(args):
         sim.sync()
         ms = e0.elapsed_time(e1)
         out[prec] = dict(mlups=round(sim.N * args.steps / (ms * 1e-3) / 1e6, 1),
-                         bytes_per_node=BYTES_PER_NODE[prec],
+                         bytes_per_node=bytes_per_node(
+                             prec, sim.N, P.auto_ordering(sim.N, n, prec)),
                          num_node=sim.N, device_bytes=sim.info()["device_bytes"])
         sim.close()
     flag, _, _ = P.sphere_pack_device(2, n, n, n, 8.0, 8.0, 0.20)
