@@ -682,7 +682,7 @@ static cudaError_t step_chain(plb_batch *b, bool grouped, int grid,
     const int bt = b->cta;
     const void *fn = batch_step_kernel(b->precision, false, bt, grid, b->shorts);
     const void *fn_m = batch_step_kernel(b->precision, true, bt, grid, b->shorts);
-    const int smem = batch_step_smem(b->precision, bt, grid, b->shorts);
+    a.trigger = batch_step_trigger(b->precision, bt, grid, b->shorts);
     args.assign((size_t)b->K, a);
     nodes.assign((size_t)b->K, nullptr);
     cudaGraph_t g = nullptr;
@@ -701,7 +701,6 @@ static cudaError_t step_chain(plb_batch *b, bool grouped, int grid,
         p.func = (void *)(k == b->K - 1 ? fn_m : fn);
         p.gridDim = dim3((unsigned)(grid > 0 ? grid : 1));
         p.blockDim = dim3((unsigned)bt);
-        p.sharedMemBytes = (unsigned)smem;
         p.kernelParams = kp;
         e = cudaGraphAddKernelNode(&nodes[(size_t)k], g, nullptr, 0, &p);
         /* each step starts while the one before drains (pdl_wait) */
@@ -818,17 +817,17 @@ static int set_chain_grid(plb_batch *b, cudaGraphExec_t exec, std::vector<BatchA
     const int bt = b->cta;
     const void *fn = batch_step_kernel(b->precision, false, bt, grid, b->shorts);
     const void *fn_m = batch_step_kernel(b->precision, true, bt, grid, b->shorts);
-    const int smem = batch_step_smem(b->precision, bt, grid, b->shorts);
+    const int trigger = batch_step_trigger(b->precision, bt, grid, b->shorts);
     const int pf = chain_prefetch(b, grid);
     for (int k = 0; k < b->K; k++) {
         args[(size_t)k].pf_blocks = pf;
+        args[(size_t)k].trigger = trigger;
         void *kp[1] = {&args[(size_t)k]};
         cudaKernelNodeParams p;
         memset(&p, 0, sizeof(p));
         p.func = (void *)(k == b->K - 1 ? fn_m : fn);
         p.gridDim = dim3((unsigned)grid);
         p.blockDim = dim3((unsigned)bt);
-        p.sharedMemBytes = (unsigned)smem;
         p.kernelParams = kp;
         BCK(cudaGraphExecKernelNodeSetParams(exec, nodes[(size_t)k], &p));
     }

@@ -198,11 +198,16 @@ struct StepArgs {
     int pf_blocks;           /* L2 prefetch distance in blocks (0 = none) */
     int words_first;         /* the FP64 form's kernels, built for both, load
                                 the words before the wait */
+    int trigger;             /* Trigger */
 };
 
 /* How a step kernel reads its words: whole ones after the wait for the step
  * before, or before it (see words_first_waves); short ones (before it). */
 enum WordMode { kWordsLate, kWordsFirst, kWordsShort };
+
+/* Where a step lets the next one's CTAs start (they then wait for this step to
+ * complete): see step_trigger. */
+enum Trigger { kTriggerStart, kTriggerWaited, kTriggerGathered, kTriggerExit };
 
 /* Waves of resident CTAs up to which a step loads its words before it waits
  * for the step before; above it, the gathers go out as their words arrive.
@@ -247,6 +252,7 @@ struct BatchArgs {
                                   max |stored deviation| */
     unsigned int *serr;        /* per-sample error bits */
     int pf_blocks;             /* L2 prefetch distance in CTAs (0 = none) */
+    int trigger;               /* Trigger */
     /* L2 groups: when grp is set, the launch steps group *grp_cur only,
      * pool blocks blk_list[grp[2g] .. grp[2g] + grp[2g + 1]) */
     const int *grp;
@@ -296,7 +302,7 @@ struct StepLaunch {
     int variant;     /* register budget (plb_params.kernel_variant) */
     int wave;        /* CTAs resident on the device at once (0: not planned) */
     int words;       /* WordMode */
-    int smem;        /* shared memory that spreads the grid over the SMs */
+    int trigger;     /* Trigger */
 };
 
 /* default threads per CTA of the step on n nodes (current device) */
@@ -320,8 +326,8 @@ int batch_default_cta(int precision);
  * another size. */
 constexpr int kBatchBlock = 256;
 const void *batch_step_kernel(int precision, bool macros, int cta, int grid, bool shorts);
-/* its shared memory (see spread_smem) */
-int batch_step_smem(int precision, int cta, int grid, bool shorts);
+/* its Trigger */
+int batch_step_trigger(int precision, int cta, int grid, bool shorts);
 
 /* Fill the coefficients from tau, F and the storage scale. */
 void make_coeffs(double tau, double force, float scale, Coeffs *c);

@@ -1104,6 +1104,7 @@ int plb_step_async(plb_sim *s, int it_begin, int nsteps)
     a.shorts = s->shorts;
     a.plane = s->plane;
     a.words_first = s->shape.words == kWordsFirst;
+    a.trigger = s->shape.trigger;
     a.pf_blocks = prefetch_ctas(s->precision, s->n, s->shape.wave, false,
                                 s->shorts != nullptr, s->prefetch);
     for (int k = 0; k < nsteps; k++) {

@@ -76,10 +76,39 @@ __device__ __forceinline__ void pdl_launch_next()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-__device__ __forceinline__ void pdl_wait()
+__device__ __forceinline__ void pdl_wait(bool launch)
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (launch) pdl_launch_next();
 }
+
+/* A kernel's share of the rule in step_trigger.  Only the FP32 and 16-bit
+ * forms' kernels for short launches can trigger after their gathers: the
+ * trigger is a point that no load is moved across, and one that does not even
+ * run costs the FP64 pool 5% and FP32 at 96^3 10%.  Where a kernel's launches
+ * all take one place it is fixed (a choice costs the 16-bit forms 2-4%): the
+ * start in these forms' long launches, after the gathers in the 16-bit forms'
+ * short ones outside pools. */
+template <int PREC, int W, bool POOL> struct TriggerPlace {
+    static constexpr bool half = PREC == PLB_FP16DEV || PREC == PLB_BF16DEV;
+    static constexpr bool dev = half || PREC == PLB_FP32;
+    static constexpr bool early = dev && (W == kWordsLate || (W == kWordsShort && !POOL));
+    static constexpr bool late = dev && W == kWordsFirst;
+    static constexpr bool fixed_late = late && half && !POOL;
+    static __device__ __forceinline__ void start(int t)
+    {
+        if (early || (!fixed_late && t == kTriggerStart)) pdl_launch_next();
+    }
+    static __device__ __forceinline__ bool waited(int t)
+    {
+        return !early && !fixed_late &&
+               (t == kTriggerWaited || (!late && t == kTriggerGathered));
+    }
+    static __device__ __forceinline__ void gathered(int t)
+    {
+        if (fixed_late || (late && t == kTriggerGathered)) pdl_launch_next();
+    }
+};
 
 /* word_at() for the form that stores T (FP32 alone has short words) */
 template <typename T>
@@ -127,18 +156,20 @@ __device__ __forceinline__ void gather(const T *fin, const uint32_t *nbr,
 
 /* The streamed values of node i (if valid), after the step before: WF loads
  * the neighbour words before the wait, else each gather goes out as its word
- * arrives after it (words_first_waves). */
+ * arrives after it (words_first_waves); `launch` triggers the next step's
+ * launch after the wait. */
 template <typename T, bool WF>
 __device__ __forceinline__ void stream_node(const void *fin, const uint32_t *nbr,
-                                            long long np, long long i, bool valid, T (&f)[Q])
+                                            long long np, long long i, bool valid, bool launch,
+                                            T (&f)[Q])
 {
     if constexpr (WF) {
         int w[Q - 1];
         if (valid) load_words<T>(nbr, np, i, w);
-        pdl_wait();
+        pdl_wait(launch);
         if (valid) gather_words<T>((const T *)fin, np, i, w, f);
     } else {
-        pdl_wait();
+        pdl_wait(launch);
         if (valid) gather<T>((const T *)fin, nbr, np, i, f);
     }
 }
@@ -629,14 +660,16 @@ k_step(const StepArgs a)
                                                   blockDim.x);
     using T = typename StoreOf<PREC>::T;
     T raw[Q];
-    pdl_launch_next();
+    using Trig = TriggerPlace<PREC, W, false>;
+    const bool launch = Trig::waited(a.trigger);
+    Trig::start(a.trigger);
     if constexpr (PREC == PLB_FP64) {
         /* one kernel for both: built apart, the form with the words after
          * the wait spills 20 B at its 128 registers (348 against 341 us at
          * 256^3); FP32 and 16-bit kernels are the ones with registers to
          * lose to a branch */
-        if (a.words_first) stream_node<T, true>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
-        else stream_node<T, false>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
+        if (a.words_first) stream_node<T, true>(a.fin, a.nbr, a.npad, i, i < a.n, launch, raw);
+        else stream_node<T, false>(a.fin, a.nbr, a.npad, i, i < a.n, launch, raw);
     } else if constexpr (W == kWordsShort) {
         /* the short words are asked for before it is known whether the block
          * has them: a block that has not (1 in 60) reads 36 bytes a node
@@ -647,14 +680,15 @@ k_step(const StepArgs a)
             load_short(a.nbr, i, q);
             is_short = __ldg(a.shorts + (i >> 8)) != 0;
         }
-        pdl_wait();
+        pdl_wait(launch);
         if (i < a.n) {
             if (is_short) gather_short<T>((const T *)a.fin, q, a.npad, i, a.plane, a.n, raw);
             else gather<T>((const T *)a.fin, a.nbr, a.npad, i, raw);
         }
     } else {
-        stream_node<T, W == kWordsFirst>(a.fin, a.nbr, a.npad, i, i < a.n, raw);
+        stream_node<T, W == kWordsFirst>(a.fin, a.nbr, a.npad, i, i < a.n, launch, raw);
     }
+    Trig::gathered(a.trigger);
     double sum_u = 0.0, sum_r = 0.0;
     if (i < a.n) {
         float dm = 0.f;
@@ -738,7 +772,9 @@ k_batch_step(const BatchArgs a)
      * block maps and words above and below are the interval's: no step
      * writes them, so they are read before the wait (see k_step) */
     T raw[Q];
-    pdl_launch_next();
+    using Trig = TriggerPlace<PREC, W, true>;
+    const bool launch = Trig::waited(a.trigger);
+    Trig::start(a.trigger);
     if (W == kWordsShort && a.shorts[pb]) {
         uint32_t q[9];
         int plane = 0;
@@ -746,11 +782,12 @@ k_batch_step(const BatchArgs a)
             load_short(a.nbr, i, q);
             plane = a.samples[s].plane;
         }
-        pdl_wait();
+        pdl_wait(launch);
         if (valid) gather_short<T>((const T *)a.fin, q, a.npad, i, plane, a.rest, raw);
     } else {
-        stream_node<T, W == kWordsFirst>(a.fin, a.nbr, a.npad, i, valid, raw);
+        stream_node<T, W == kWordsFirst>(a.fin, a.nbr, a.npad, i, valid, launch, raw);
     }
+    Trig::gathered(a.trigger);
     if (valid) {
         {
             /* the sample's coefficients straight from global memory (the
@@ -807,14 +844,13 @@ k_batch_step(const BatchArgs a)
 
 /* One step launch, overlapping the kernel before it in the stream (see
  * pdl_wait). */
-static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, int smem,
-                              const StepArgs &a, cudaStream_t s)
+static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, const StepArgs &a,
+                              cudaStream_t s)
 {
     cudaLaunchConfig_t c;
     memset(&c, 0, sizeof(c));
     c.gridDim = dim3((unsigned)grid);
     c.blockDim = dim3((unsigned)block);
-    c.dynamicSmemBytes = (size_t)smem;
     c.stream = s;
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -822,47 +858,6 @@ static cudaError_t launch_pdl(void (*fn)(StepArgs), int grid, int block, int sme
     c.attrs = &at;
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, fn, a);
-}
-
-/* Shared memory a step CTA asks for (and does not use) so that an SM holds
- * no more CTAs than an even spread of the grid gives it.  While a step's
- * CTAs start among the last of the step before, the free SMs take several
- * each and the rest none: at 16k to 76k nodes a step then took up to twice
- * its time (at 16k nodes FP64 5.4 against 3.0 us, FMA form 27 / 7.7; FP32 at
- * 76k 4.1 / 2.8).  The requests only cap the residency; a grid that needs every CTA slot of an SM keeps all of its L1
- * (FP32 at 179k nodes: 4.3 us, capped 4.8).  0 = no cap. */
-template <typename Fn>
-static int spread_smem(Fn fn, Fn fn_macros, int grid, int block)
-{
-    int dev = 0, sms = 0, per = 0, total = 0, reserved = 0, most = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) !=
-            cudaSuccess ||
-        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) !=
-            cudaSuccess ||
-        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)fn, block, 0) !=
-            cudaSuccess ||
-        sms <= 0 || grid <= 0)
-        return 0;
-    const int share = (grid + sms - 1) / sms;
-    if (share >= per) return 0;
-    /* the macro kernels' own static shared memory (under 1 KB) comes on top */
-    const int slack = 1024;
-    int smem = (total / share - reserved - slack) / 1024 * 1024;
-    if (smem > most - slack) smem = most - slack;
-    /* the same limit whatever the grid: handles of other sizes and threads
-     * set it too */
-    if (cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             most - slack) != cudaSuccess ||
-        cudaFuncSetAttribute((const void *)fn_macros, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             most - slack) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return smem;
 }
 
 template <int PREC, int V>
@@ -897,8 +892,7 @@ static cudaError_t launch_prec(bool macros, const StepArgs &a, const StepLaunch 
 {
     const int grid = (a.n + l.block - 1) / l.block;
     if (grid == 0) return cudaSuccess;
-    return launch_pdl(step_variant<PREC>(macros, l.words, l.variant), grid, l.block,
-                      l.smem, a, s);
+    return launch_pdl(step_variant<PREC>(macros, l.words, l.variant), grid, l.block, a, s);
 }
 
 /* CTAs of a kernel resident on an SM of the current device, and its SMs;
@@ -909,6 +903,35 @@ static bool occupancy(const void *fn, int block, int *per, int *sms)
     return cudaGetDevice(&dev) == cudaSuccess &&
            cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
            cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, fn, block, 0) == cudaSuccess;
+}
+
+/* Where a step of `grid` CTAs of `block` threads, `per` of them to an SM,
+ * lets the next step's CTAs start: at once where the launch fills the device.
+ * In a shorter one the CTAs of the steps after would pile up on the SMs that
+ * are free first, several of one step on an SM and none on others, and a step
+ * take up to twice its time (FMA form at 46k nodes 30 against 20 us, FP64 at
+ * 38k 6.1 against 3.8, FP32 at 39k 3.3 against 2.2).  There
+ *   FP32, 16-bit  after the gathers (FP32 at 92k nodes 3.0 us, right after the
+ *                 wait 3.8); in a pool of few CTAs, which reads its block maps
+ *                 first, right after the wait (FP16, 76k nodes: 2.6 / 3.4)
+ *   FP64 forms    right after the wait while an SM has a CTA or two; more of
+ *                 them keep it busy for long enough that the next step's have
+ *                 to find it free: at this step's end (bit-exact at 61k nodes
+ *                 17.7 us, after the wait 23.5; FP64 at 22k 4.1 / 3.7)
+ * An alternative, CTAs that ask for so much shared memory that an SM holds no
+ * more than its share, is as fast (92k nodes FP32 3.3 us, FP16 2.75) but keeps
+ * other handles off the device: eight FP32 handles of 92k nodes then take 43
+ * us for a step each, and 28 without. */
+static int step_trigger(int precision, bool pool, long long grid, int block, int per, int sms)
+{
+    const long long share = (grid + sms - 1) / sms; /* CTAs of an SM */
+    if (precision == PLB_FP64_EXACT || precision == PLB_FP64 || precision == PLB_FP64_FMA) {
+        if (share > per) return kTriggerStart;
+        const long long few = precision == PLB_FP64_FMA ? 128 : 256; /* threads */
+        return grid * block > few * sms && share < per ? kTriggerExit : kTriggerWaited;
+    }
+    if (share >= per) return kTriggerStart;
+    return pool && share <= 3 && share * block <= 512 ? kTriggerWaited : kTriggerGathered;
 }
 
 /* L2 bytes of the current device, 0 if unknown */
@@ -973,9 +996,9 @@ static void plan_prec(int n, StepLaunch *l)
     l->wave = occupancy((const void *)step_variant<PREC>(false, kWordsLate, l->variant), l->block,
                         &per, &sms) ? sms * per : 0;
     l->words = grid <= words_first_waves(PREC) * (long long)l->wave ? kWordsFirst : kWordsLate;
-    l->smem = spread_smem(step_variant<PREC>(false, l->words, l->variant),
-                          step_variant<PREC>(true, l->words, l->variant), grid,
-                          l->block);
+    l->trigger = occupancy((const void *)step_variant<PREC>(false, l->words, l->variant), l->block,
+                           &per, &sms) ? step_trigger(PREC, false, grid, l->block, per, sms)
+                                       : kTriggerStart;
 }
 
 void plan_step(int precision, int n, StepLaunch *l)
@@ -1089,13 +1112,6 @@ static const void *batch_fn_cta(bool macros, int cta, int grid, bool shorts)
                       : batch_fn<PREC, kBatchBlock>(macros, words);
 }
 
-int batch_step_smem(int precision, int cta, int grid, bool shorts)
-{
-    const void *fn = batch_step_kernel(precision, false, cta, grid, shorts);
-    const void *fn_m = batch_step_kernel(precision, true, cta, grid, shorts);
-    return fn && fn_m ? spread_smem(fn, fn_m, grid, cta) : 0;
-}
-
 const void *batch_step_kernel(int precision, bool macros, int cta, int grid, bool shorts)
 {
     if (cta != 128 && cta != kBatchBlock) return nullptr;
@@ -1108,6 +1124,14 @@ const void *batch_step_kernel(int precision, bool macros, int cta, int grid, boo
     case PLB_BF16DEV: return batch_fn_cta<PLB_BF16DEV>(macros, cta, grid, shorts);
     default: return nullptr;
     }
+}
+
+int batch_step_trigger(int precision, int cta, int grid, bool shorts)
+{
+    int per = 0, sms = 0;
+    const void *fn = batch_step_kernel(precision, false, cta, grid, shorts);
+    return fn && occupancy(fn, cta, &per, &sms) ? step_trigger(precision, true, grid, cta, per, sms)
+                                                : kTriggerStart;
 }
 
 cudaError_t launch_step(int precision, bool macros, const StepArgs &a, const StepLaunch &l,
