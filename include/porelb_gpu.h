@@ -79,13 +79,14 @@ enum {
  * in one shifted run of nodes, which gathers best while the three z-planes
  * a step reads at once stay in L2.  MORTON keeps the gathers local at any
  * size.  AUTO takes REFERENCE when three z-planes of the domain's nodes
- * (their distributions, words and numbering) fit in 60% of the L2, else
- * MORTON
- * (256^3: row order, FP64 17.2 against 16.4 GLUPS; 512^3 FP16 and FP32 up to
- * 1024^3: row order; 512^3 and 1024^3 FP64: Morton). */
+ * (their distributions, words and numbering) fit in 60% of the L2 or, where
+ * FP32's 16-bit words fit the domain (they do but for planes of a few very
+ * long rows), in 1.75 times the L2; else MORTON (256^3, 512^3 FP16 and FP32 up
+ * to 1024^3: row order; 512^3 and 1024^3 FP64: Morton). */
 enum { PLB_ORDER_MORTON = 0, PLB_ORDER_REFERENCE = 1, PLB_ORDER_AUTO = 2 };
 /* The order AUTO picks for n nodes in an nx*ny*nz domain with elem-byte
- * storage on device `device`. */
+ * storage on device `device` (4-byte storage: where 16-bit words fit; the
+ * order a handle has is plb_words's). */
 int plb_auto_ordering(long long n, int nz, int elem_bytes, int device);
 
 /* Wall rule. */
@@ -263,6 +264,11 @@ int plb_kernel_flags(plb_sim *sim, unsigned *flags);
 int plb_info(plb_sim *sim, int *num_node, int *npad, int *precision,
              size_t *device_bytes);
 void *plb_stream(plb_sim *sim);
+/* How the handle keeps its nodes: their order (PLB_ORDER_MORTON or
+ * PLB_ORDER_REFERENCE), the blocks of 256 nodes, and those of them whose
+ * neighbour words are 16 bits wide (FP32 domains that outgrow the L2: a step
+ * reads 36 bytes of words a node instead of 72).  Any pointer may be NULL. */
+int plb_words(plb_sim *sim, int *ordering, int *blocks, int *short_blocks);
 
 /* ---------------------------------------------------------------- batch */
 
@@ -365,6 +371,8 @@ int plb_batch_info(plb_batch *b, long long *t, int *active,
                    long long *used_nodes, long long *capacity_nodes,
                    size_t *device_bytes);
 int plb_batch_sample_nodes(plb_batch *b, int id, int *num_node);
+/* A sample's 256-node pool blocks and those with 16-bit neighbour words. */
+int plb_batch_sample_words(plb_batch *b, int id, int *blocks, int *short_blocks);
 /* Room left in the pool, in nodes: the largest free block range (0 when no
  * sample slot is free) and all free ranges together.  A sample of n fluid
  * nodes can be admitted now when ceil(n / 256) * 256 <= *largest_range. */

@@ -95,6 +95,7 @@ _SIGS = {
     "plb_permeability": (_I, [_P, _DP, _DP]),
     "plb_last_error": (_I, [_P, _IP, _IP, _IP, _IP, _IP, _DP]),
     "plb_info": (_I, [_P, _IP, _IP, _IP, ctypes.POINTER(ctypes.c_size_t)]),
+    "plb_words": (_I, [_P, _IP, _IP, _IP]),
     "plb_stream": (_P, [_P]),
     "plb_status_string": (ctypes.c_char_p, [_I]),
     "plb_batch_bytes_per_node": (ctypes.c_size_t, [_I, _I]),
@@ -125,6 +126,7 @@ _SIGS = {
     "plb_kernel_flags": (_I, [_P, ctypes.POINTER(ctypes.c_uint)]),
     "plb_get_f_streamed": (_I, [_P, _P]),
     "plb_batch_sample_nodes": (_I, [_P, _I, _IP]),
+    "plb_batch_sample_words": (_I, [_P, _I, _IP, _IP]),
     "plb_batch_free_nodes": (_I, [_P, ctypes.POINTER(ctypes.c_longlong),
                                   ctypes.POINTER(ctypes.c_longlong)]),
     "plb_batch_stream": (_P, [_P]),

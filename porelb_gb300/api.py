@@ -144,7 +144,8 @@ def _params(tau, force, precision, ordering, halo, block_size, device,
 def auto_ordering(num_node, nz, precision, device=0):
     """The node order PLB_ORDER_AUTO picks for this domain and form:
     "reference" (row order) when three z-planes of its nodes fit in 60% of
-    the L2 (FP32: in 1.75 times the L2), else "morton"."""
+    the L2 (FP32, where 16-bit words fit: in 1.75 times the L2), else
+    "morton".  Simulation.words() has the order of a handle."""
     elem = {"fp64_exact": 8, "fp64": 8, "fp64_fma": 8, "fp32": 4, "fp16dev": 2,
             "bf16dev": 2}[precision]
     o = _lib.load().plb_auto_ordering(int(num_node), int(nz), elem, device)
@@ -284,6 +285,15 @@ class Simulation:
                                   ctypes.byref(prec), ctypes.byref(b)), "info")
         return dict(num_node=n.value, npad=npad.value, precision=prec.value,
                     device_bytes=b.value)
+
+    def words(self):
+        """The handle's node order, its blocks of 256 nodes and how many of
+        those have 16-bit neighbour words (36 bytes a node instead of 72)."""
+        o, b, s = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+        _check(self._lib.plb_words(self._h, ctypes.byref(o), ctypes.byref(b),
+                                   ctypes.byref(s)), "words")
+        return dict(ordering="reference" if o.value == _lib.ORDER_REFERENCE else "morton",
+                    blocks=b.value, short_blocks=s.value)
 
     @classmethod
     def _from_handle(cls, h, nx, ny, nz, tau, force, precision):

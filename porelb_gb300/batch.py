@@ -174,6 +174,14 @@ class Batch:
                "sample_nodes")
         return n.value
 
+    def sample_words(self, sid):
+        """A sample's pool blocks of 256 nodes and how many of them have
+        16-bit neighbour words."""
+        b, s = ctypes.c_int(), ctypes.c_int()
+        _check(self._lib.plb_batch_sample_words(self._h, sid, ctypes.byref(b),
+                                                ctypes.byref(s)), "sample_words")
+        return dict(blocks=b.value, short_blocks=s.value)
+
     def get_f(self, sid):
         out = np.empty(self.num_nodes(sid) * _lib.Q)
         _check(self._lib.plb_batch_get_f(self._h, sid, _ptr(out)), "get_f")

@@ -188,7 +188,7 @@ __global__ void k_get_macro_sample(const double *macro, long long npad, long lon
 }
 
 /* a sample's node table moved into another pool: pull words re-based */
-__global__ void k_translate_words(const uint32_t *src, const uint8_t *sshorts, int plane,
+__global__ void k_translate_words(const uint32_t *src, const int2 *sshorts,
                                   long long srows, long long snp, long long sbase, uint32_t srest,
                                   uint32_t *dst, long long drows, long long dnp, long long dbase,
                                   uint32_t drest, int n)
@@ -199,7 +199,7 @@ __global__ void k_translate_words(const uint32_t *src, const uint8_t *sshorts, i
 #pragma unroll
     for (int j = 1; j < Q; j++) {
         const uint32_t w =
-            (uint32_t)word_of(src, sshorts, j, sbase + k, srows, snp, plane, (int)srest);
+            (uint32_t)word_of(src, sshorts, j, sbase + k, srows, snp, (int)srest);
         uint32_t o;
         if (w == srest) o = drest;
         else if ((long long)(uint32_t)(w - (uint32_t)sbase) < (long long)n)
@@ -265,7 +265,7 @@ struct plb_batch {
     void *f[2] = {nullptr, nullptr};
     int cur = 0;
     uint32_t *nbr = nullptr;
-    uint8_t *shorts = nullptr; /* pool blocks with short words (forms that read them) */
+    int2 *shorts = nullptr; /* by pool block: short words (forms that read them) */
     int *perm = nullptr;
     uint16_t *coord = nullptr;
     double *macro = nullptr;
@@ -447,7 +447,7 @@ int plb_batch_create_ex(const plb_batch_params *bp, plb_batch **out)
     al(&b->nbr, 4 * word_count(precision, b->npad));
     /* L2 groups step inside the L2, where short words only cost */
     if (short_words_pay(precision, b->rest) && !b->group_bytes)
-        al(&b->shorts, (size_t)b->npad / kWordNodes);
+        al(&b->shorts, sizeof(int2) * ((size_t)b->npad / kWordNodes));
     al(&b->perm, 4 * np);
     al(&b->coord, 2 * 3 * np);
     if (keep_macros) al(&b->macro, 8 * 4 * np);
@@ -465,7 +465,7 @@ int plb_batch_create_ex(const plb_batch_params *bp, plb_batch **out)
     if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_serr, 4 * (size_t)max_samples);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->blk, 0xff, 4 * (size_t)b->cap_blocks, b->st);
     if (e == cudaSuccess && b->shorts)
-        e = cudaMemsetAsync(b->shorts, 0, (size_t)b->npad / kWordNodes, b->st);
+        e = cudaMemsetAsync(b->shorts, 0x80, sizeof(int2) * ((size_t)b->npad / kWordNodes), b->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->sactive, 0, 4 * (size_t)max_samples, b->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->serr, 0, 4 * (size_t)max_samples, b->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->t_dev, 0, 4, b->st);
@@ -546,14 +546,14 @@ static int add_dflag(plb_batch *b, const GeomWork &w, int nx, int ny, int nz,
     if (rc == PLB_OK) {
         const long long base = blk0 * B;
         const int order = b->ordering == PLB_ORDER_AUTO
-                              ? plb_auto_ordering(n, nz, (int)b->elem, b->device)
+                              ? auto_order(n, nz, (int)b->elem, b->shorts != nullptr, b->device)
                               : b->ordering;
         rc = flag_tables(w, nx, ny, nz, 1, order, 0, 0, n, b->npad, b->perm + base, b->coord + base,
                          b->nbr, word_rows(b->precision, b->npad), (uint32_t)base, (uint32_t)b->rest,
                          b->adm);
         if (rc == PLB_OK && b->shorts &&
-            shorten_words(b->nbr, b->shorts, base, n, n / nz, (int)b->rest, true, nullptr,
-                          b->adm) != cudaSuccess)
+            shorten_words(b->nbr, b->shorts, base, n, (int)b->rest, true, nullptr, b->adm) !=
+                cudaSuccess)
             rc = PLB_ERR_CUDA;
         if (rc != PLB_OK) free_range(b, blk0, nblk);
     }
@@ -587,7 +587,6 @@ static int add_dflag(plb_batch *b, const GeomWork &w, int nx, int ny, int nz,
     make_coeffs(sp->tau, sp->force_x, h.scale, &d.co);
     d.base = blk0 * B;
     d.n = n;
-    d.plane = n / nz;
     /* a sample admitted while an interval runs starts after it */
     d.start = (int)(b->t + (b->in_flight ? b->K : 0));
     h.start = d.start;
@@ -1134,12 +1133,12 @@ int plb_batch_transfer(plb_batch *src, int id, plb_batch *dst, int *new_id)
                                 2 * (size_t)n, cudaMemcpyDeviceToDevice, dst->adm);
         if (e == cudaSuccess) {
             k_translate_words<<<gb(n, B), B, 0, dst->adm>>>(
-                src->nbr, src->shorts, hs.dev.plane, word_rows(src->precision, src->npad),
+                src->nbr, src->shorts, word_rows(src->precision, src->npad),
                 src->npad, sb, (uint32_t)src->rest, dst->nbr,
                 word_rows(dst->precision, dst->npad), dst->npad, db, (uint32_t)dst->rest, n);
             if (dst->shorts)
-                e = shorten_words(dst->nbr, dst->shorts, db, n, n / hs.nz, (int)dst->rest, true,
-                                  nullptr, dst->adm);
+                e = shorten_words(dst->nbr, dst->shorts, db, n, (int)dst->rest, true, nullptr,
+                                  dst->adm);
             switch (src->precision) {
             case PLB_FP32: convert_to<float>(src, hs, dst, db, scale); break;
             case PLB_FP16DEV: convert_to<__half>(src, hs, dst, db, scale); break;
@@ -1173,7 +1172,6 @@ int plb_batch_transfer(plb_batch *src, int id, plb_batch *dst, int *new_id)
     make_coeffs(h.tau, h.force, h.scale, &d.co);
     d.base = db;
     d.n = n;
-    d.plane = n / h.nz;
     d.start = (int)h.start;
     BCK(cudaMemcpyAsync(dst->sdev + sid, &d, sizeof(d), cudaMemcpyHostToDevice, dst->adm));
     BCK(cudaMemsetAsync(dst->serr + sid, 0, 4, dst->adm));
@@ -1326,6 +1324,25 @@ int plb_batch_interval_ms(plb_batch *b, float *ms)
 {
     if (!b || !ms) return PLB_ERR_ARG;
     *ms = b->last_ms;
+    return PLB_OK;
+}
+
+int plb_batch_sample_words(plb_batch *b, int id, int *blocks, int *short_blocks)
+{
+    if (!b || id < 0 || id >= b->max_samples || !b->s[id].used) return PLB_ERR_ARG;
+    const SampleHost &h = b->s[id];
+    const int m = (h.n + B - 1) / B;
+    int count = 0;
+    if (b->shorts && m > 0) {
+        BCK(cudaSetDevice(b->device));
+        std::vector<int2> at((size_t)m);
+        BCK(cudaMemcpyAsync(at.data(), b->shorts + h.blk0, sizeof(int2) * (size_t)m,
+                            cudaMemcpyDeviceToHost, b->adm));
+        BCK(cudaStreamSynchronize(b->adm));
+        for (const int2 &x : at) count += x.x != kWholeWords;
+    }
+    if (blocks) *blocks = m;
+    if (short_blocks) *short_blocks = count;
     return PLB_OK;
 }
 

@@ -226,46 +226,78 @@ __global__ void k_nbr_from_flag(const TableArgs a)
 
 /* One CTA per block of 256 nodes; see shorten_words. */
 __global__ void __launch_bounds__(kWordNodes)
-k_shorten_words(uint32_t *nbr, uint8_t *shorts, long long lo, int n, int plane, int rest,
-                int rewrite, int *count)
+k_shorten_words(uint32_t *nbr, int2 *shorts, long long lo, int n, int rest, int rewrite, int *count)
 {
+    __shared__ int least[3], most[3]; /* distances, by dz_planes() + 1 */
     const long long blk = (lo >> 8) + blockIdx.x;
     const long long i = blk * kWordNodes + threadIdx.x;
-    bool fits = true;
+    if (threadIdx.x < 3) {
+        least[threadIdx.x] = 0x7fffffff;
+        most[threadIdx.x] = -0x7fffffff;
+    }
+    __syncthreads();
+    int a[3] = {0x7fffffff, 0x7fffffff, 0x7fffffff};
+    int b[3] = {-0x7fffffff, -0x7fffffff, -0x7fffffff};
+    if (i < lo + n) {
+#pragma unroll
+        for (int j = 1; j < Q; j++) {
+            const int s = (int)nbr[word_at(j, i, 0)];
+            if (s == rest || s < lo || s >= lo + n) continue;
+            const int d = s - (int)i, z = dz_planes(j) + 1;
+            a[z] = min(a[z], d);
+            b[z] = max(b[z], d);
+        }
+    }
+#pragma unroll
+    for (int z = 0; z < 3; z++) {
+        const int l = __reduce_min_sync(0xffffffffu, a[z]), m = __reduce_max_sync(0xffffffffu, b[z]);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&least[z], l);
+            atomicMax(&most[z], m);
+        }
+    }
+    __syncthreads();
+    /* those to another plane count from the smallest (none: from 0) */
+    const int2 base = make_int2(least[2] > most[2] ? 0 : least[2],
+                                least[0] > most[0] ? 0 : least[0]);
+    constexpr int kMost = (int)kShortBounce - 1; /* the largest distance kept */
+    const bool all = (least[2] > most[2] || most[2] - least[2] <= kMost) &&
+                     (least[0] > most[0] || most[0] - least[0] <= kMost) &&
+                     (least[1] > most[1] ||
+                      (least[1] >= -kShortBias && most[1] <= kMost - kShortBias));
+    if (threadIdx.x == 0) {
+        shorts[blk] = all ? base : make_int2(kWholeWords, 0);
+        if (all && count) atomicAdd(count, 1);
+    }
+    if (!all || !rewrite) return;
     uint32_t q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     if (i < lo + n) {
 #pragma unroll
         for (int j = 1; j < Q; j++) {
             const int s = (int)nbr[word_at(j, i, 0)];
-            long long d = kShortBounce;
-            if (s == rest) {
-                d = kShortRest;
-            } else if (s >= lo && s < lo + n) {
-                d = s - i - (long long)dz_planes(j) * plane + kShortBias;
-                fits = fits && d >= 0 && d < kShortBounce;
-            }
-            q[(j - 1) >> 1] |= ((uint32_t)d & 0xffffu) << ((j & 1) ? 0 : 16);
+            uint32_t d = kShortBounce;
+            if (s == rest) d = kShortRest;
+            else if (s >= lo && s < lo + n)
+                d = (uint32_t)(s - (int)i - (dz_planes(j) == 0  ? -kShortBias
+                                             : dz_planes(j) > 0 ? base.x
+                                                                : base.y));
+            q[(j - 1) >> 1] |= d << ((j & 1) ? 0 : 16);
         }
     }
     /* every word of the block has been read when the first is rewritten */
-    const bool all = __syncthreads_and(fits);
-    if (threadIdx.x == 0) {
-        shorts[blk] = (uint8_t)all;
-        if (all && count) atomicAdd(count, 1);
-    }
-    if (!all || !rewrite) return;
+    __syncthreads();
     uint32_t *p = nbr + blk * kWordBlock;
     ((uint4 *)p)[threadIdx.x] = make_uint4(q[0], q[1], q[2], q[3]);
     ((uint4 *)p)[256 + threadIdx.x] = make_uint4(q[4], q[5], q[6], q[7]);
     p[2048 + threadIdx.x] = q[8];
 }
 
-cudaError_t shorten_words(uint32_t *nbr, uint8_t *shorts, long long lo, int n, int plane,
-                          int rest, bool rewrite, int *count, cudaStream_t st)
+cudaError_t shorten_words(uint32_t *nbr, int2 *shorts, long long lo, int n, int rest,
+                          bool rewrite, int *count, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
     k_shorten_words<<<(unsigned)((n + kWordNodes - 1) / kWordNodes), kWordNodes, 0, st>>>(
-        nbr, shorts, lo, n, plane, rest, rewrite, count);
+        nbr, shorts, lo, n, rest, rewrite, count);
     return cudaGetLastError();
 }
 

@@ -91,15 +91,21 @@ __host__ __device__ constexpr long long word_at(int j, long long i, long long ro
     return rows ? word_in_rows(j, i, rows) : word_in_block(j, i);
 }
 
-/* Short words.  In row order the sources of direction j lie close to i +
- * dz_planes(j) * plane, with plane the domain's mean nodes per z-plane.  A
- * block of 256 nodes whose sources all lie within 16 bits of that keeps its
- * words as 16-bit distances instead, in the first half of its place: two rows
- * of eight and one of two.  Two more values mean the node's own reversed
- * value and the rest slot.  All blocks but those at the periodic wraps fit
- * (98-99% at 128^3 to 400^3), and a step of the FP32 form, which streams at
- * the copy rate, reads 36 bytes a node less (256^3: 190 -> 163 us, 36 GLUPS). */
-constexpr int kShortBias = 32767; /* distance d is kept as d + kShortBias */
+/* Short words.  In row order the sources of direction j lie close to the node
+ * itself (dz_planes(j) == 0) or to the node's place in the next or the last
+ * z-plane, a distance that is nearly the same for neighbouring nodes.  A block
+ * of 256 nodes whose sources all lie within 16 bits of those keeps its words
+ * as 16-bit distances instead, in the first half of its place: two rows of
+ * eight and one of two.  Two more values mean the node's own reversed value
+ * and the rest slot.  Each block has its own two plane distances (what they are counted from),
+ * so it makes no difference how much the planes' node counts vary; what does
+ * not fit are rows at a periodic wrap in y of planes of more than 32k nodes,
+ * and Morton order.  A step of the FP32 form, which streams at the copy rate,
+ * reads 36 bytes a node less (256^3: 190 -> 163 us, 36 GLUPS). */
+constexpr int kShortBias = 32767; /* a distance d in the plane: d + kShortBias */
+/* The distance that a block's words count from for dz_planes(j) == 1 (x) and
+ * -1 (y), its smallest; x = kWholeWords for a block whose words are whole. */
+constexpr int kWholeWords = -0x7f7f7f80; /* every byte 0x80 */
 constexpr uint32_t kShortBounce = 0xfffe;
 constexpr uint32_t kShortRest = 0xffff;
 __host__ __device__ constexpr int dz_planes(int j) { return -ez(j); }
@@ -141,26 +147,26 @@ __device__ __forceinline__ void load_short(const uint32_t *nbr, long long i, uin
 
 /* the pull word of direction j that node i's short words stand for */
 __device__ __forceinline__ int short_word(const uint32_t (&q)[9], int j, int i, long long npad,
-                                          int plane, int rest)
+                                          int2 base, int rest)
 {
     const uint32_t pair = q[(j - 1) >> 1];
     const bool high = !(j & 1);
     const uint32_t w = high ? pair >> 16 : pair & 0xffffu;
-    int o = (i + dz_planes(j) * plane - kShortBias) + (int)w;
+    const int from = dz_planes(j) == 0 ? -kShortBias : (dz_planes(j) > 0 ? base.x : base.y);
+    int o = (i + from) + (int)w;
     if (high ? pair >= (kShortBounce << 16) : w >= kShortBounce) o = i + (opp(j) - j) * (int)npad;
     if (high ? pair >= (kShortRest << 16) : w >= kShortRest) o = rest;
     return o;
 }
 
 /* the pull word of direction j of node i, whichever way its block is kept */
-__device__ __forceinline__ int word_of(const uint32_t *nbr, const uint8_t *shorts, int j,
-                                       long long i, long long rows, long long npad, int plane,
-                                       int rest)
+__device__ __forceinline__ int word_of(const uint32_t *nbr, const int2 *shorts, int j,
+                                       long long i, long long rows, long long npad, int rest)
 {
-    if (!shorts || !shorts[i >> 8]) return (int)nbr[word_at(j, i, rows)];
+    if (!shorts || shorts[i >> 8].x == kWholeWords) return (int)nbr[word_at(j, i, rows)];
     uint32_t q[9];
     load_short(nbr, i, q);
-    return short_word(q, j, (int)i, npad, plane, rest);
+    return short_word(q, j, (int)i, npad, shorts[i >> 8], rest);
 }
 #endif
 
@@ -183,8 +189,7 @@ struct StepArgs {
     const void *fin;
     void *fout;
     const uint32_t *nbr;  /* word_at() */
-    const uint8_t *shorts; /* blocks of 256 nodes with short words; may be NULL */
-    int plane;             /* mean nodes per z-plane (short words) */
+    const int2 *shorts;   /* by block of 256 nodes (see kWholeWords); may be NULL */
     int rest;              /* the rest slot */
     const int *perm;      /* new -> reference index (density guard report) */
     long long npad;
@@ -229,14 +234,13 @@ struct SampleDev {
     long long base; /* first node of the sample in the pool */
     int n;          /* fluid nodes */
     int start;      /* batch step at which the sample started */
-    int plane;      /* mean nodes per z-plane (short words) */
 };
 
 struct BatchArgs {
     const void *fin;
     void *fout;
     const uint32_t *nbr;
-    const uint8_t *shorts;     /* pool blocks with short words; may be NULL */
+    const int2 *shorts;        /* by pool block (see kWholeWords); may be NULL */
     int rest;                  /* the rest slot */
     long long npad;
     const int *blk_list;       /* pool blocks this launch covers (one CTA each,
@@ -288,10 +292,13 @@ int flag_tables(const GeomWork &w, int nx, int ny, int nz, int num_p, int orderi
                 cudaStream_t st);
 
 /* Short words for the blocks of nodes lo .. lo + n - 1 (lo a multiple of 256)
- * whose sources are near: flags the blocks in shorts, counts them in *count
+ * whose sources are near: fills in the blocks' shorts, counts them in *count
  * (device memory, may be NULL) and, with `rewrite`, rewrites their words. */
-cudaError_t shorten_words(uint32_t *nbr, uint8_t *shorts, long long lo, int n, int plane,
-                          int rest, bool rewrite, int *count, cudaStream_t st);
+cudaError_t shorten_words(uint32_t *nbr, int2 *shorts, long long lo, int n, int rest,
+                          bool rewrite, int *count, cudaStream_t st);
+
+/* the node order for n nodes (plb_auto_ordering), with short words or without */
+int auto_order(long long n, int nz, int elem_bytes, bool shorts, int device);
 
 /* whether `nodes` nodes step faster with short words */
 bool short_words_pay(int precision, long long nodes);

@@ -43,9 +43,10 @@ struct plb_sim {
     int cur;
     size_t elem;
     uint32_t *nbr;
-    uint8_t *shorts;  /* blocks with short words; NULL = none */
-    uint8_t *shorts_mem;
-    int plane;        /* mean nodes per z-plane */
+    int2 *shorts;     /* by block: short words; NULL = none */
+    int2 *shorts_mem;
+    int short_blocks; /* blocks with short words */
+    bool row_if_short; /* AUTO took row order for the sake of short words */
     int *perm;        /* new -> reference index */
     uint16_t *coord;  /* [3][npad] x, y, z in new order */
     double *macro;    /* [4][npad] */
@@ -77,11 +78,9 @@ struct plb_sim {
 
 /* ------------------------------------------------------ ordering */
 
-int plb_auto_ordering(long long n, int nz, int elem_bytes, int device)
+int plb::auto_order(long long n, int nz, int elem_bytes, bool shorts, int device)
 {
-    /* bytes a step moves per node: 19 values in and out, 18 words (short ones
-     * in the form that has them), perm */
-    const bool shorts = elem_bytes == 4;
+    /* bytes a step moves per node: 19 values in and out, 18 words, perm */
     const double bpn = 2.0 * 19 * elem_bytes + (shorts ? 36 : 72) + 4;
     int l2 = 0;
     if (nz <= 0 || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device) != cudaSuccess ||
@@ -90,11 +89,18 @@ int plb_auto_ordering(long long n, int nz, int elem_bytes, int device)
     const double plane = bpn * (double)n / nz;
     /* measured: row order wins up to about 63 MB of such planes on a 126 MB
      * L2 (512^3 FP16) and loses from 105 MB (512^3 FP64, whose L2 prefetch
-     * also takes room).  FP32 keeps short words in row order only: 35.9
+     * also takes room; FP32 with whole words, 1024 x 1024 x 48, at 287 MB).
+     * FP32 keeps short words in row order only: 35.9
      * against 30.3 GLUPS at 30 MB (512^3, porosity 0.2), 34.9 / 30.5 at 121
      * (1024^3), 32.1 / 30.3 at 211 (1024^3, porosity 0.35), the largest
      * measured */
-    return 3.0 * plane <= (shorts ? 1.75 : 0.6) * (double)l2 ? PLB_ORDER_REFERENCE : PLB_ORDER_MORTON;
+    return 3.0 * plane <= (shorts ? 1.75 : 0.6) * (double)l2 ? PLB_ORDER_REFERENCE
+                                                             : PLB_ORDER_MORTON;
+}
+
+int plb_auto_ordering(long long n, int nz, int elem_bytes, int device)
+{
+    return auto_order(n, nz, elem_bytes, elem_bytes == 4, device);
 }
 
 /* ------------------------------------------------------ allocation */
@@ -555,16 +561,16 @@ __global__ void k_get_f_dev(const T *f, const int *perm, long long npad, int n,
 
 /* the next step's streamed values (through the pull words), FP64 AoS */
 template <typename T>
-__global__ void k_get_streamed(const T *f, const uint32_t *nbr, const uint8_t *shorts, int plane,
-                               long long rows, const int *perm, long long npad, int n, float inv_scale,
-                               double *out)
+__global__ void k_get_streamed(const T *f, const uint32_t *nbr, const int2 *shorts,
+                               long long rows, const int *perm, long long npad, int n,
+                               float inv_scale, double *out)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const long long o = (long long)perm[k] * Q;
 #pragma unroll
     for (int j = 0; j < Q; j++) {
-        const long long at = j == 0 ? k : (long long)j * npad + word_of(nbr, shorts, j, k, rows, npad, plane, n);
+        const long long at = j == 0 ? k : (long long)j * npad + word_of(nbr, shorts, j, k, rows, npad, n);
         if constexpr (sizeof(T) == 8) {
             out[o + j] = ((const double *)f)[at];
         } else {
@@ -803,9 +809,11 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
     s->num_p = num_p;
     s->npad = ((long long)n + 1 + 63) / 64 * 64;
     s->precision = p->precision;
-    s->ordering = p->ordering == PLB_ORDER_AUTO
-                      ? plb_auto_ordering(n, nz, (int)elem_size(p->precision), p->device)
-                      : p->ordering;
+    const int elem = (int)elem_size(p->precision);
+    s->ordering = p->ordering == PLB_ORDER_AUTO ? plb_auto_ordering(n, nz, elem, p->device)
+                                                : p->ordering;
+    s->row_if_short = p->ordering == PLB_ORDER_AUTO && s->ordering == PLB_ORDER_REFERENCE &&
+                      auto_order(n, nz, elem, false, p->device) == PLB_ORDER_MORTON;
     s->halo = p->halo;
     s->boundary = p->boundary;
     /* register budget of the step kernel (kernel_variant 1 and 3 are the
@@ -844,7 +852,7 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
     } part[] = {{&s->f[0], fbytes},
                 {&s->f[1], fbytes},
                 {(void **)&s->nbr, 4 * word_count(s->precision, s->npad)},
-                {(void **)&s->shorts_mem, (np + kWordNodes - 1) / kWordNodes},
+                {(void **)&s->shorts_mem, sizeof(int2) * ((np + kWordNodes - 1) / kWordNodes)},
                 {(void **)&s->perm, 4 * np},
                 {(void **)&s->coord, 2 * 3 * np},
                 {(void **)&s->macro, 8 * 4 * np},
@@ -871,14 +879,14 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
         return e == cudaErrorMemoryAllocation ? PLB_ERR_NOMEM : PLB_ERR_CUDA;
     }
     s->dev_bytes = acc;
-    s->plane = n / nz;
     plan_step(s->precision, n, &s->shape);
     *out = s;
     return PLB_OK;
 }
 
-/* Short words where they pay and most blocks fit: nearly all do in row order,
- * none in Morton order, whose words stay wide.  The words are read once to
+/* Short words where they pay and three blocks in four fit (a block that does
+ * not reads 36 bytes a node too many): nearly all do in row order, seldom so
+ * many in Morton order, whose words then stay whole.  The words are read once to
  * count and once to rewrite them: 0.06 ms of a creation at 128^3 (of 0.47),
  * 0.26 ms at 256^3 (of 1.29), what ten to twenty steps gain. */
 static cudaError_t make_short_words(plb_sim *s)
@@ -888,20 +896,37 @@ static cudaError_t make_short_words(plb_sim *s)
     int h = 0;
     cudaError_t e = cudaMemsetAsync(count, 0, 4, s->stream);
     if (e == cudaSuccess)
-        e = shorten_words(s->nbr, s->shorts_mem, 0, s->n, s->plane, s->n, false, count, s->stream);
+        e = shorten_words(s->nbr, s->shorts_mem, 0, s->n, s->n, false, count, s->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, count, 4, cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    if (e != cudaSuccess || 2LL * h * kWordNodes < s->n) return e;
+    if (e != cudaSuccess || 4LL * h * kWordNodes < 3LL * s->n) return e;
     s->shorts = s->shorts_mem;
+    s->short_blocks = h;
     s->shape.words = kWordsShort;
-    return shorten_words(s->nbr, s->shorts, 0, s->n, s->plane, s->n, true, nullptr, s->stream);
+    return shorten_words(s->nbr, s->shorts, 0, s->n, s->n, true, nullptr, s->stream);
+}
+
+/* The tables by build() in the handle's order, with short words where they
+ * pay; a row order that AUTO took for their sake gives way to Morton where
+ * they do not fit (planes past 0.6 of the L2: 1024 x 1024 x 64 with whole words
+ * 852 us a step in row order, 773 in Morton). */
+template <typename Build>
+static int make_tables(plb_sim *s, Build build)
+{
+    int rc = build();
+    if (rc != PLB_OK) return rc;
+    if (make_short_words(s) != cudaSuccess) return PLB_ERR_CUDA;
+    if (s->row_if_short && !s->shorts) {
+        s->ordering = PLB_ORDER_MORTON;
+        rc = build();
+    }
+    return rc;
 }
 
 static int sim_finish(plb_sim *s, int rc, plb_sim **out)
 {
     if (rc == PLB_OK) {
-        cudaError_t e = make_short_words(s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(s->err, 0xff, 8, s->stream);
+        cudaError_t e = cudaMemsetAsync(s->err, 0xff, 8, s->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(s->flags, 0, 4, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) rc = PLB_ERR_CUDA;
@@ -930,7 +955,7 @@ int plb_create(const plb_node_info *V, int num_node, int nx, int ny, int nz,
     plb_sim *s = nullptr;
     int rc = sim_alloc(p, num_node, nx, ny, nz, num_p, v_sub_start, &s);
     if (rc != PLB_OK) return rc;
-    return sim_finish(s, build_tables(s, V), out);
+    return sim_finish(s, make_tables(s, [&] { return build_tables(s, V); }), out);
 }
 
 /* Tables from the flag grid in w. */
@@ -947,11 +972,14 @@ static int create_from_dflag(const GeomWork &w, int nx, int ny, int nz,
     if (rc == PLB_OK) {
         const int remote_wins = (s->halo == PLB_HALO_REMOTE_WINS) ||
                                 (s->halo == PLB_HALO_AUTO && s->num_p > 1);
-        rc = flag_tables(w, nx, ny, nz, num_p, s->ordering, remote_wins,
-                         s->boundary, n, s->npad, s->perm, s->coord,
-                         s->nbr, word_rows(s->precision, s->npad), 0u, (uint32_t)n, st);
-        if (rc == PLB_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = PLB_ERR_CUDA;
-        rc = sim_finish(s, rc, out);
+        auto build = [&] {
+            int e = flag_tables(w, nx, ny, nz, num_p, s->ordering, remote_wins, s->boundary, n,
+                                s->npad, s->perm, s->coord, s->nbr,
+                                word_rows(s->precision, s->npad), 0u, (uint32_t)n, st);
+            if (e == PLB_OK && cudaStreamSynchronize(st) != cudaSuccess) e = PLB_ERR_CUDA;
+            return e;
+        };
+        rc = sim_finish(s, make_tables(s, build), out);
     }
     free(slab);
     return rc;
@@ -1102,7 +1130,6 @@ int plb_step_async(plb_sim *s, int it_begin, int nsteps)
     a.err = s->err;
     a.flags = s->flags;
     a.shorts = s->shorts;
-    a.plane = s->plane;
     a.words_first = s->shape.words == kWordsFirst;
     a.trigger = s->shape.trigger;
     a.pf_blocks = prefetch_ctas(s->precision, s->n, s->shape.wave, false,
@@ -1283,10 +1310,10 @@ int plb_get_f_streamed(plb_sim *s, double *f_aos)
     switch (s->precision) {
     case PLB_FP64_EXACT:
     case PLB_FP64:
-    case PLB_FP64_FMA: k_get_streamed<double><<<g, 256, 0, s->stream>>>((const double *)f, s->nbr, s->shorts, s->plane, rows, s->perm, s->npad, s->n, inv, d); break;
-    case PLB_FP32: k_get_streamed<float><<<g, 256, 0, s->stream>>>((const float *)f, s->nbr, s->shorts, s->plane, rows, s->perm, s->npad, s->n, inv, d); break;
-    case PLB_FP16DEV: k_get_streamed<__half><<<g, 256, 0, s->stream>>>((const __half *)f, s->nbr, s->shorts, s->plane, rows, s->perm, s->npad, s->n, inv, d); break;
-    default: k_get_streamed<__nv_bfloat16><<<g, 256, 0, s->stream>>>((const __nv_bfloat16 *)f, s->nbr, s->shorts, s->plane, rows, s->perm, s->npad, s->n, inv, d); break;
+    case PLB_FP64_FMA: k_get_streamed<double><<<g, 256, 0, s->stream>>>((const double *)f, s->nbr, s->shorts, rows, s->perm, s->npad, s->n, inv, d); break;
+    case PLB_FP32: k_get_streamed<float><<<g, 256, 0, s->stream>>>((const float *)f, s->nbr, s->shorts, rows, s->perm, s->npad, s->n, inv, d); break;
+    case PLB_FP16DEV: k_get_streamed<__half><<<g, 256, 0, s->stream>>>((const __half *)f, s->nbr, s->shorts, rows, s->perm, s->npad, s->n, inv, d); break;
+    default: k_get_streamed<__nv_bfloat16><<<g, 256, 0, s->stream>>>((const __nv_bfloat16 *)f, s->nbr, s->shorts, rows, s->perm, s->npad, s->n, inv, d); break;
     }
     cudaError_t e = cudaGetLastError();
     host_populate(f_aos, bytes);
@@ -1373,6 +1400,15 @@ int plb_info(plb_sim *s, int *num_node, int *npad, int *precision,
     if (npad) *npad = (int)s->npad;
     if (precision) *precision = s->precision;
     if (device_bytes) *device_bytes = s->dev_bytes;
+    return PLB_OK;
+}
+
+int plb_words(plb_sim *sim, int *ordering, int *blocks, int *short_blocks)
+{
+    if (!sim) return PLB_ERR_ARG;
+    if (ordering) *ordering = sim->ordering;
+    if (blocks) *blocks = (sim->n + kWordNodes - 1) / kWordNodes;
+    if (short_blocks) *short_blocks = sim->short_blocks;
     return PLB_OK;
 }
 

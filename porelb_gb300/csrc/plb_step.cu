@@ -177,12 +177,12 @@ __device__ __forceinline__ void stream_node(const void *fin, const uint32_t *nbr
 /* the streamed values of node i from its short words q */
 template <typename T>
 __device__ __forceinline__ void gather_short(const T *fin, const uint32_t (&q)[9], long long np,
-                                             long long i, int plane, int rest, T (&f)[Q])
+                                             long long i, int2 base, int rest, T (&f)[Q])
 {
     f[0] = fin[i];
 #pragma unroll
     for (int j = 1; j < Q; j++)
-        f[j] = fin[(long long)j * np + short_word(q, j, (int)i, np, plane, rest)];
+        f[j] = fin[(long long)j * np + short_word(q, j, (int)i, np, base, rest)];
 }
 
 /* ------------------------------------------------- FP64, reference order */
@@ -617,7 +617,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes)
  * bytes inside its row or its word block. */
 template <typename T>
 __device__ __forceinline__ void prefetch_block(const T *fin, const uint32_t *nbr,
-                                               const uint8_t *shorts, long long np, long long n,
+                                               const int2 *shorts, long long np, long long n,
                                                long long b, int bs)
 {
     const long long i0 = b * bs;
@@ -630,7 +630,7 @@ __device__ __forceinline__ void prefetch_block(const T *fin, const uint32_t *nbr
         long long end = i0 + cnt;
         if (sizeof(T) == 4 && (k | 255) + 1 < end) end = (k | 255) + 1;
         const unsigned m = (unsigned)(end - k);
-        if (shorts && shorts[k >> 8]) {
+        if (shorts && shorts[k >> 8].x != kWholeWords) {
             const uint32_t *p = nbr + (k >> 8) * kWordBlock;
             prefetch_l2(p + 4 * (k & 255), m * 16);
             prefetch_l2(p + 1024 + 4 * (k & 255), m * 16);
@@ -675,14 +675,14 @@ k_step(const StepArgs a)
          * has them: a block that has not (1 in 60) reads 36 bytes a node
          * for nothing, the others wait for one load less */
         uint32_t q[9];
-        bool is_short = false;
+        int2 base = make_int2(0, 0);
         if (i < a.n) {
             load_short(a.nbr, i, q);
-            is_short = __ldg(a.shorts + (i >> 8)) != 0;
+            base = __ldg(a.shorts + (i >> 8));
         }
         pdl_wait(launch);
         if (i < a.n) {
-            if (is_short) gather_short<T>((const T *)a.fin, q, a.npad, i, a.plane, a.n, raw);
+            if (base.x != kWholeWords) gather_short<T>((const T *)a.fin, q, a.npad, i, base, a.n, raw);
             else gather<T>((const T *)a.fin, a.nbr, a.npad, i, raw);
         }
     } else {
@@ -775,15 +775,13 @@ k_batch_step(const BatchArgs a)
     using Trig = TriggerPlace<PREC, W, true>;
     const bool launch = Trig::waited(a.trigger);
     Trig::start(a.trigger);
-    if (W == kWordsShort && a.shorts[pb]) {
+    int2 base = make_int2(kWholeWords, 0);
+    if (W == kWordsShort) base = a.shorts[pb];
+    if (W == kWordsShort && base.x != kWholeWords) {
         uint32_t q[9];
-        int plane = 0;
-        if (valid) {
-            load_short(a.nbr, i, q);
-            plane = a.samples[s].plane;
-        }
+        if (valid) load_short(a.nbr, i, q);
         pdl_wait(launch);
-        if (valid) gather_short<T>((const T *)a.fin, q, a.npad, i, plane, a.rest, raw);
+        if (valid) gather_short<T>((const T *)a.fin, q, a.npad, i, base, a.rest, raw);
     } else {
         stream_node<T, W == kWordsFirst>(a.fin, a.nbr, a.npad, i, valid, launch, raw);
     }
