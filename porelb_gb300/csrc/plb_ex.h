@@ -31,9 +31,12 @@
  * integer-to-FP64 conversion: about 65 of a node's 260.
  *
  * Domain (anything else is reported and the caller takes another path):
- * f_0 in [1/4, 3/4), f_1..6 in [2^-7, 3/32), f_7..18 in [2^-8, 3/64), rho in
- * [1/2, 5/4), |u_a| < 0.08, omega + a in [1/8, 2), and 1 - omega zero or of
- * magnitude >= 2^-40.
+ * f_0 in [1/4, 1), f_1..6 in [2^-7, 2^-3), f_7..18 in [2^-8, 2^-4), rho in
+ * [1/2, 1.2], |u_a| < 0.11, omega + a in [1/8, 2) for every direction (or,
+ * for a large tau, in a range 16 times as wide from its lower end to its upper
+ * that is a power of two lower), and 1 - omega zero or of magnitude >= 2^-40.
+ * A node that is outside by its velocity alone is told apart: its moments
+ * stand.
  *
  * Measured (256^3 pack, 5.87M nodes): 992 us a step (5.9 GLUPS) against 2204
  * (2.66) with every add on the FP64 pipe and IEEE products made one by one
@@ -125,7 +128,7 @@ EX_HD uint64_t rne(uint64_t v, uint32_t d)
 }
 
 /* a * b / 2^64 rounded to nearest even at 53 significant bits, in place, for
- * a product in [2^118, 2^127) and (a >> 32) + (b >> 32) < 2^32 (which keeps
+ * a product in [2^117, 2^127) and (a >> 32) + (b >> 32) < 2^32 (which keeps
  * the sum of the middle products below 2^64).  The 64 bits below enter as
  * one: with the kept part's last bit they decide a tie. */
 EX_HD uint64_t mulr(uint64_t a, uint64_t b)
@@ -211,6 +214,7 @@ struct Consts {
     uint64_t om;   /* |1 - omega|'s significand, in [2^62, 2^63); 0 if omega = 1 */
     uint32_t omsh; /* |1 - omega| = om * 2^(-61 - ash - omsh) */
     uint32_t ash;  /* the forcing factor and the results are scaled 2^ash higher */
+    uint32_t up;   /* the forcing factor is scaled 2^up higher still (TINY) */
     uint32_t neg;  /* 1 if 1 - omega < 0 */
     uint32_t ok;   /* the run's constants lie in the domain: 1, or 2 for TINY */
 };
@@ -234,12 +238,24 @@ static inline Consts make_consts(double omega, double om1, double k3, double for
     if (k.ok && k.omsh > 5u) k.ok = 2u;
     /* the forcing factor's bounds for any node (each node checks its own);
      * tau > 2.5 has 1 - omega in [0.6, 1): two places up fit */
-    const double far = 1.08 * fabs(k3 * force);
+    const double far = 1.11 * fabs(k3 * force);
     if (omega + far < 0.4) {
         k.ash = 2u;
         k.omsh -= 2u;
     }
-    if (!(omega - far >= (k.ash ? 0.03125 : 0.125) && omega + far < 2.0)) k.ok = 0u;
+    if (k.ok && k.ash && !(omega - far >= 0.03125)) {
+        /* tau > 32: the factor with its own scale, its product shifted back.
+         * (1 - omega) f is whole at the two places that are left, so the
+         * sticky one of the sum is the product's alone */
+        k.ok = 2u;
+        k.omsh += k.ash;
+        k.ash = 0u;
+        while (k.up < 40u && omega + far < ldexp(1.0, -(int)k.up)) k.up++;
+        if (!(omega - far >= ldexp(0.125, -(int)k.up) && omega + far < ldexp(2.0, -(int)k.up)))
+            k.ok = 0u;
+    } else if (!(omega - far >= (k.ash ? 0.03125 : 0.125) && omega + far < 2.0)) {
+        k.ok = 0u;
+    }
     k.neg = om1 < 0.0;
     return k;
 }
@@ -310,10 +326,13 @@ struct Out {
 
 /* One collision.  b[19]: post-stream FP64 bits; store(j, bits) receives each
  * post-collision value as it is made (holding them to the end would cost the
- * registers of a third of the warps).  Returns nonzero when the node lies
- * outside the domain; store may then have received some values.  TINY:
- * |1 - omega| < 1/16, whose products can lose bits in the class scale and
- * leave a sticky one. */
+ * registers of a third of the warps).  Returns kOutside or kFast when the node
+ * lies outside the domain; store may then have received some values.  kFast:
+ * o holds the moments all the same.  TINY: |1 - omega| < 1/16, whose products
+ * can lose bits in the class scale and leave a sticky one, or k.up > 0, whose
+ * products with the forcing factor can. */
+constexpr uint32_t kOutside = 1u, kFast = 2u;
+
 template <bool TINY, typename Store>
 EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Out &o,
                        const Store &store)
@@ -327,9 +346,9 @@ EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Ou
         if (xc(j) == 1) { lo1 = umin(lo1, h); hi1 = umax(hi1, h); }
         else { lo2 = umin(lo2, h); hi2 = umax(hi2, h); }
     }
-    uint32_t outside = (uint32_t)(hi32(b[0]) - 0x3fd00000u >= 0x180000u) |
-                       (uint32_t)(lo1 < 0x3f800000u) | (uint32_t)(hi1 >= 0x3fb80000u) |
-                       (uint32_t)(lo2 < 0x3f700000u) | (uint32_t)(hi2 >= 0x3fa80000u);
+    uint32_t outside = (uint32_t)(hi32(b[0]) - 0x3fd00000u >= 0x200000u) |
+                       (uint32_t)(lo1 < 0x3f800000u) | (uint32_t)(hi1 >= 0x3fc00000u) |
+                       (uint32_t)(lo2 < 0x3f700000u) | (uint32_t)(hi2 >= 0x3fb00000u);
     uint64_t F[Q]; /* class scale */
     F[0] = scaled<0>(b[0]);
 #pragma unroll
@@ -356,9 +375,10 @@ EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Ou
             jmax = imax(jmax, (int32_t)hi32((uint64_t)J[a]));
         }
     }
-    outside |= (uint32_t)(S - ((uint64_t)1 << 60) >= ((uint64_t)3 << 59)); /* [1/2, 5/4) */
-    if (outside) return 1u;
-    o.bad = (uint32_t)(S > 0x2666666666666600ull); /* 1.2 */
+    /* [1/2, 1.2], which is the density guard's range */
+    outside |= (uint32_t)(S - ((uint64_t)1 << 60) > 0x1666666666666600ull);
+    if (outside) return kOutside;
+    o.bad = 0u;
 
     /* momentum: exact when every partial sum is below 2^-5 and a multiple of
      * 2^-58, else native adds */
@@ -404,14 +424,13 @@ EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Ou
     o.v = v;
     o.w = w;
     {
-        /* |u| < 0.08; j_x (the force's share can be any number) zero or far
+        /* |u| < 0.11; j_x (the force's share can be any number) zero or far
          * from underflow */
         const uint32_t hu = hi32(bits_of(u)) & 0x7fffffffu, hv = hi32(bits_of(v)) & 0x7fffffffu,
                        hw = hi32(bits_of(w)) & 0x7fffffffu;
         const uint64_t jx = bits_of(m[0]) << 1;
-        outside = (uint32_t)(umax(umax(hu, hv), hw) >= 0x3fb47ae1u) |
-                  (uint32_t)(jx != 0ull && hi32(jx) < (128u << 20));
-        if (outside) return 1u;
+        if (jx != 0ull && hi32(jx) < (128u << 20)) return kOutside;
+        if (umax(umax(hu, hv), hw) >= 0x3fbc28f5u) return kFast;
     }
 
     const double uv = add(add(mul(u, u), mul(v, v)), mul(w, w));
@@ -429,11 +448,12 @@ EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Ou
             const double d = e == 0 ? -u : sub((double)e, u);
             const double a = add(k.omega, mul(mul(k.k3, d), k.force));
             const uint64_t ab = bits_of(a);
-            outside |= (uint32_t)(hi32(ab) - ((1020u - k.ash) << 20) >= (4u << 20));
-            A[e + 1] = mant(ab) << (expo(ab) + k.ash - 1013u & 63u);
+            const uint32_t s = TINY ? k.ash + k.up : k.ash;
+            outside |= (uint32_t)(hi32(ab) - ((1020u - s) << 20) >= (4u << 20));
+            A[e + 1] = mant(ab) << (expo(ab) + s - 1013u & 63u);
         }
     }
-    if (outside) return 1u;
+    if (outside) return kFast;
 
     uint32_t rmin = ~0u, rmax = 0;
     const uint64_t flip = (uint64_t)0 - k.neg;
@@ -441,6 +461,7 @@ EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Ou
     auto relax = [&](int j, uint64_t T, uint64_t hc, uint64_t a) {
         /* feq * 2^(61 + s), the rest * 2^(59 + s + ash) */
         uint64_t R = mulr(a, mulr(hc, T));
+        if (TINY) R = shr_odd(R, k.up);
         if (k.om != 0ull) {
             uint64_t p = mulr(k.om, F[j]);
             p = TINY ? shr_odd(p, k.omsh) : shr(p, k.omsh);
@@ -476,9 +497,11 @@ EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Ou
         eu = of_bits(bits_of(eu) & 0x7fffffffffffffffull);
         const uint64_t t3 = q62_triple(eu);
         const uint64_t c2 = q62(mul(mul(4.5, eu), eu));
-        /* plus: 1 + t3 and + c2 are >= 1 (last place 2^-52); minus: both
-         * <= 1 (2^-53), since 4.5 eu^2 < 3 |eu|; - 1.5 u.u can bring the
-         * plus one below 1 */
+        /* plus: 1 + t3 and + c2 are in [1, 2) (last place 2^-52); minus: 1 - t3
+         * is exact where t3 >= 1/2, and then + c2 and - 1.5 u.u stay in
+         * [1/2, 1] (2^-53), since 4.5 eu^2 < 3 |eu| and 1 - 6 a + 15 a^2 -
+         * 1.5 a^2 > 1/2 for a < 0.111; - 1.5 u.u can bring the plus one below
+         * 1 */
         const uint64_t p = kOne + rne(rne(t3, 10u) + c2, 10u) - uv15;
         const uint64_t n = kOne - rne(t3, 9u) + c2;
         const uint64_t Tp = rne(p, 9u + (hi32(p) >> 30));
@@ -488,6 +511,7 @@ EX_HD uint32_t collide(const uint64_t (&b)[19], const Consts &k, bool it_pos, Ou
     }
     /* exact integers convert whatever their size and sign, but zero; with a
      * sticky one they have to keep two bits below the last place */
+    static_assert(kOutside == 1u, "");
     return TINY ? (uint32_t)(rmin < (1u << 24)) | (uint32_t)(rmax >= (1u << 28))
                 : (uint32_t)(rmin == 0u);
 }

@@ -234,31 +234,12 @@ struct Macro {
     bool bad;
 };
 
-template <bool NATIVE>
-__device__ __forceinline__ Macro collide_fp64_exact(double (&f)[Q],
-                                                     const Coeffs &a, uint32_t &outside)
+/* The collision from a node's moments (u shifted by the force): f(j) gives
+ * the streamed values, store(j, x) takes the others. */
+template <bool NATIVE, typename Value, typename Store>
+__device__ __forceinline__ void relax_fp64_exact(const Coeffs &a, double rho, double u, double v,
+                                                 double w, const Value &f, const Store &store)
 {
-    Macro m;
-    double rho = f[0];
-#pragma unroll
-    for (int j = 1; j < Q; j++) rho = dadd(rho, f[j]);
-    double ru = moment_ref<0>(f);
-    const double rv = moment_ref<1>(f);
-    const double rw = moment_ref<2>(f);
-    m.bad = (rho > 1.2) | (rho < 0.5);
-    if constexpr (!NATIVE) {
-        /* the density in [2^-64, 2^64) too, or the node takes the native
-         * multiply (the caller) */
-        const uint64_t rb = (uint64_t)__double_as_longlong(rho);
-        outside |= emu::outside_node_range(rb) | (uint32_t)((rb << 1) == 0ull);
-        if (outside) return m;
-    }
-    if (a.it > 0) ru = dadd(ru, a.half_force);
-    const double u = __ddiv_rn(ru, rho);
-    const double v = __ddiv_rn(rv, rho);
-    const double w = __ddiv_rn(rw, rho);
-    m.rho = rho; m.u = u; m.v = v; m.w = w;
-
     const double uv = dadd(dadd(dmul(u, u), dmul(v, v)), dmul(w, w));
     const double uv15 = dmul(1.5, uv);
     const double h0 = dmul(w64(0), rho);
@@ -272,7 +253,7 @@ __device__ __forceinline__ Macro collide_fp64_exact(double (&f)[Q],
     /* rest direction: e.u = 0 gives ((1 + 0) + 0) - 1.5 uv */
     {
         const double feq = imul<NATIVE>(h0, dsub(1.0, uv15));
-        f[0] = dadd(imul<NATIVE>(a.om1, f[0]), imul<NATIVE>(a0, feq));
+        store(0, dadd(imul<NATIVE>(a.om1, f(0)), imul<NATIVE>(a0, feq)));
     }
     /* pairs (J, J+1) with e_{J+1} = -e_J: 3 e.u, 4.5 e.u and (4.5 e.u) e.u
      * of the partner are exact negations / the same value. */
@@ -295,9 +276,37 @@ __device__ __forceinline__ Macro collide_fp64_exact(double (&f)[Q],
         const double feqK = imul<NATIVE>(h, dsub(dadd(dsub(1.0, t3), c2), uv15));
         const double AJ = ex(J) > 0 ? ap : (ex(J) < 0 ? am : a0);
         const double AK = ex(K) > 0 ? ap : (ex(K) < 0 ? am : a0);
-        f[J] = dadd(imul<NATIVE>(a.om1, f[J]), imul<NATIVE>(AJ, feqJ));
-        f[K] = dadd(imul<NATIVE>(a.om1, f[K]), imul<NATIVE>(AK, feqK));
+        store(J, dadd(imul<NATIVE>(a.om1, f(J)), imul<NATIVE>(AJ, feqJ)));
+        store(K, dadd(imul<NATIVE>(a.om1, f(K)), imul<NATIVE>(AK, feqK)));
     }
+}
+
+template <bool NATIVE>
+__device__ __forceinline__ Macro collide_fp64_exact(double (&f)[Q],
+                                                     const Coeffs &a, uint32_t &outside)
+{
+    Macro m;
+    double rho = f[0];
+#pragma unroll
+    for (int j = 1; j < Q; j++) rho = dadd(rho, f[j]);
+    double ru = moment_ref<0>(f);
+    const double rv = moment_ref<1>(f);
+    const double rw = moment_ref<2>(f);
+    m.bad = (rho > 1.2) | (rho < 0.5);
+    if constexpr (!NATIVE) {
+        /* the density in [2^-64, 2^64) too, or the node takes the native
+         * multiply (the caller) */
+        const uint64_t rb = (uint64_t)__double_as_longlong(rho);
+        outside |= emu::outside_node_range(rb) | (uint32_t)((rb << 1) == 0ull);
+        if (outside) return m;
+    }
+    if (a.it > 0) ru = dadd(ru, a.half_force);
+    m.rho = rho;
+    m.u = __ddiv_rn(ru, rho);
+    m.v = __ddiv_rn(rv, rho);
+    m.w = __ddiv_rn(rw, rho);
+    relax_fp64_exact<NATIVE>(a, rho, m.u, m.v, m.w, [&](int j) { return f[j]; },
+                             [&](int j, double x) { f[j] = x; });
     return m;
 }
 
@@ -482,13 +491,30 @@ template <int PREC, int V, int W> struct MinBlocks {
     }
 };
 
+/* The bit-exact collision of node i that left plb_ex.h's domain by its
+ * velocity, from its moments: its streamed values, gathered again, are needed
+ * one by one, and all 19 are stored again (128^3 with every node past the
+ * range: 500 us a step, from the values alone 635).  Out of line, so the common
+ * path keeps its registers. */
+__device__ __noinline__ void exact_node_fast(const double *fin, double *fout, const uint32_t *nbr,
+                                             long long np, long long i, const Coeffs *run,
+                                             double rho, double u, double v, double w)
+{
+    int at[Q - 1];
+    load_words<double>(nbr, np, i, at);
+    auto value = [&](int j) { return fin[j == 0 ? i : (long long)j * np + at[j - 1]]; };
+    auto store = [&](int j, double x) { __stcs(fout + (long long)j * np + i, x); };
+    if (run->exact_native) relax_fp64_exact<true>(*run, rho, u, v, w, value, store);
+    else relax_fp64_exact<false>(*run, rho, u, v, w, value, store);
+}
+
 /* The bit-exact collision of node i outside plb_ex.h's common domain, from
  * its streamed values gathered again, stored: plb_ex.h's form for tau within
- * 1/16 of 1; else the products on the integer pipes for a node in their
- * range, every product on the FP64 pipe for one whose values or density (or
- * the run's constants) lie outside it, such as an infinity, a NaN, a
- * subnormal or an extreme value.  Out of line, so the common path keeps its
- * registers. */
+ * 1/16 of 1 or above 32 (128^3: 192 us a step, the products' form 358); else
+ * the products on the integer pipes for a node in their range, every product
+ * on the FP64 pipe for one whose values or density (or the run's constants)
+ * lie outside it, such as an infinity, a NaN, a subnormal or an extreme value.
+ * Out of line, so the common path keeps its registers. */
 __device__ __noinline__ Macro exact_node_wide(const double *fin, double *fout,
                                               const uint32_t *nbr, long long np,
                                               long long i, const Coeffs *run, int it,
@@ -508,7 +534,11 @@ __device__ __noinline__ Macro exact_node_wide(const double *fin, double *fout,
         outside = ex_::collide<true>(b, co.exk, co.it > 0, o, [&](int j, uint64_t v) {
             __stcs(fout + (long long)j * np + i, __longlong_as_double((long long)v));
         });
-        if (!outside) {
+        if (outside == ex_::kFast) {
+            exact_node_fast(fin, fout, nbr, np, i, run, o.rho, o.u, o.v, o.w);
+            if (co.exact_native) *flags |= 2u;
+        }
+        if (outside != ex_::kOutside) {
             m.rho = o.rho; m.u = o.u; m.v = o.v; m.w = o.w;
             m.bad = o.bad != 0u;
             return m;
@@ -569,13 +599,18 @@ __device__ __forceinline__ Macro collide_node(T (&raw)[Q], const T *fin, T *fout
 #pragma unroll
         for (int j = 0; j < Q; j++) b[j] = (uint64_t)__double_as_longlong(raw[j]);
         ex_::Out o;
-        uint32_t outside = co.exk.ok ^ 1u;
+        uint32_t outside = co.exk.ok == 1u ? 0u : ex_::kOutside;
         if (!outside)
             outside = ex_::collide<false>(b, co.exk, co.it > 0, o, [&](int j, uint64_t v) {
                 __stcs(fout + (long long)j * np + i, __longlong_as_double((long long)v));
             });
-        /* it stores all 19 values again */
-        if (outside) return exact_node_wide(fin, fout, nbr, np, i, run, co.it, &flags);
+        /* these store all 19 values again */
+        if (outside == ex_::kOutside)
+            return exact_node_wide(fin, fout, nbr, np, i, run, co.it, &flags);
+        if (outside == ex_::kFast) {
+            exact_node_fast(fin, fout, nbr, np, i, run, o.rho, o.u, o.v, o.w);
+            if (co.exact_native) flags |= 2u;
+        }
         m.rho = o.rho; m.u = o.u; m.v = o.v; m.w = o.w;
         m.bad = o.bad != 0u;
     } else if constexpr (PREC == PLB_FP64_FMA) {
