@@ -195,11 +195,12 @@ __global__ void k_translate_words(const uint32_t *src, const int2 *sshorts,
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
+    int from[Q - 1];
+    words_of(src, sshorts, sbase + k, srows, snp, (int)srest, from);
     uint32_t words[Q - 1];
 #pragma unroll
     for (int j = 1; j < Q; j++) {
-        const uint32_t w =
-            (uint32_t)word_of(src, sshorts, j, sbase + k, srows, snp, (int)srest);
+        const uint32_t w = (uint32_t)from[j - 1];
         uint32_t o;
         if (w == srest) o = drest;
         else if ((long long)(uint32_t)(w - (uint32_t)sbase) < (long long)n)

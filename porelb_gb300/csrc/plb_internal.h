@@ -159,14 +159,25 @@ __device__ __forceinline__ int short_word(const uint32_t (&q)[9], int j, int i, 
     return o;
 }
 
-/* the pull word of direction j of node i, whichever way its block is kept */
-__device__ __forceinline__ int word_of(const uint32_t *nbr, const int2 *shorts, int j,
-                                       long long i, long long rows, long long npad, int rest)
+/* the pull words w[j - 1] of node i, whichever way its block is kept */
+__device__ __forceinline__ void words_of(const uint32_t *nbr, const int2 *shorts, long long i,
+                                         long long rows, long long npad, int rest, int (&w)[18])
 {
-    if (!shorts || shorts[i >> 8].x == kWholeWords) return (int)nbr[word_at(j, i, rows)];
-    uint32_t q[9];
-    load_short(nbr, i, q);
-    return short_word(q, j, (int)i, npad, shorts[i >> 8], rest);
+    if (shorts && shorts[i >> 8].x != kWholeWords) {
+        uint32_t q[9];
+        load_short(nbr, i, q);
+        const int2 base = shorts[i >> 8];
+#pragma unroll
+        for (int j = 1; j <= 18; j++) w[j - 1] = short_word(q, j, (int)i, npad, base, rest);
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int4 v = __ldg((const int4 *)(nbr + word_at(4 * q + 1, i, rows)));
+        w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+    }
+    const int2 v = __ldg((const int2 *)(nbr + word_at(17, i, rows)));
+    w[16] = v.x; w[17] = v.y;
 }
 #endif
 

@@ -568,9 +568,11 @@ __global__ void k_get_streamed(const T *f, const uint32_t *nbr, const int2 *shor
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const long long o = (long long)perm[k] * Q;
+    int w[Q - 1];
+    words_of(nbr, shorts, k, rows, npad, n, w);
 #pragma unroll
     for (int j = 0; j < Q; j++) {
-        const long long at = j == 0 ? k : (long long)j * npad + word_of(nbr, shorts, j, k, rows, npad, n);
+        const long long at = j == 0 ? k : (long long)j * npad + w[j - 1];
         if constexpr (sizeof(T) == 8) {
             out[o + j] = ((const double *)f)[at];
         } else {
