@@ -38,7 +38,7 @@ struct plb_sim {
     StepLaunch shape; /* launch shape */
     int device;
     cudaStream_t stream;
-    char *block_mem;  /* the one device block all arrays below lie in */
+    char *block_mem[2]; /* the device blocks all arrays below lie in */
     void *f[2];
     int cur;
     size_t elem;
@@ -662,7 +662,8 @@ static size_t elem_size(int precision)
 static void free_sim(plb_sim *s)
 {
     if (!s) return;
-    cudaFree(s->block_mem);
+    cudaFree(s->block_mem[0]);
+    cudaFree(s->block_mem[1]);
     if (s->stream) cudaStreamDestroy(s->stream);
     free(s->v_sub_start);
     free(s);
@@ -846,7 +847,11 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     const size_t fbytes = s->elem * Q * (size_t)s->npad;
     /* one allocation for all arrays: ten took 0.4 ms to make and 0.5 ms to
-     * free at 160^3, one takes 0.1 and 0.2 */
+     * free at 160^3, one takes 0.1 and 0.2.  A small handle's narrow arrays are
+     * a second one: allocations of up to 1 MiB share a 2 MiB page of the
+     * device, and while one lives in it those that a read-back stages in cost
+     * 5 us to make and free, not 100 (macros of 13k nodes 30 us; with all
+     * arrays in one block 130). */
     const size_t np = (size_t)s->npad;
     struct {
         void **p;
@@ -854,25 +859,27 @@ static int sim_alloc(const plb_params *p, int n, int nx, int ny, int nz,
     } part[] = {{&s->f[0], fbytes},
                 {&s->f[1], fbytes},
                 {(void **)&s->nbr, 4 * word_count(s->precision, s->npad)},
+                {(void **)&s->macro, 8 * 4 * np},
                 {(void **)&s->shorts_mem, sizeof(int2) * ((np + kWordNodes - 1) / kWordNodes)},
                 {(void **)&s->perm, 4 * np},
                 {(void **)&s->coord, 2 * 3 * np},
-                {(void **)&s->macro, 8 * 4 * np},
                 {(void **)&s->partial, 8 * 2 * (size_t)s->nblocks},
                 {(void **)&s->sums, 16},
                 {(void **)&s->err, 8},
                 {(void **)&s->flags, 4}};
-    size_t whole = 0;
-    for (auto &q : part) {
-        acc += q.bytes;
-        whole += (q.bytes + 255) / 256 * 256;
-    }
-    if (e == cudaSuccess) e = plb_cuda_malloc(&s->block_mem, whole);
-    if (e == cudaSuccess) {
-        char *at = s->block_mem;
-        for (auto &q : part) {
-            *q.p = at;
-            at += (q.bytes + 255) / 256 * 256;
+    constexpr int kParts = sizeof(part) / sizeof(part[0]);
+    const int wide = 8 * 4 * np <= (1u << 20) ? 4 : kParts; /* parts in the first block */
+    for (int b = 0, k = 0; b < 2 && e == cudaSuccess; b++) {
+        const int k0 = k, k1 = b == 0 ? wide : kParts;
+        size_t whole = 0;
+        for (k = k0; k < k1; k++) whole += (part[k].bytes + 255) / 256 * 256;
+        if (whole == 0) break;
+        e = plb_cuda_malloc(&s->block_mem[b], whole);
+        char *at = s->block_mem[b];
+        for (k = k0; k < k1 && e == cudaSuccess; k++) {
+            *part[k].p = at;
+            at += (part[k].bytes + 255) / 256 * 256;
+            acc += part[k].bytes;
         }
     }
     if (e != cudaSuccess) {
