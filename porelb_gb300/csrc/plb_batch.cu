@@ -1277,7 +1277,7 @@ int plb_batch_get_macros(plb_batch *b, int id, double *rho, double *ux,
                                                    b->perm, d);
     double *dst[4] = {rho, ux, uy, uz};
     cudaError_t e = cudaGetLastError();
-    for (int c = 0; c < 4; c++) host_populate(dst[c], 8 * (size_t)h.n);
+    host_populate_rows(dst, (size_t)h.n);
     for (int c = 0; c < 4 && e == cudaSuccess; c++)
         if (dst[c])
             e = cudaMemcpyAsync(dst[c], d + (size_t)c * h.n, 8 * (size_t)h.n,

@@ -277,6 +277,8 @@ struct BatchArgs {
 /* Make the pages of a host buffer that a device copy is about to write
  * present (plb_sim.cu). */
 void host_populate(void *p, size_t bytes);
+/* the same for four rows of n doubles (each may be NULL) */
+void host_populate_rows(double *const (&row)[4], size_t n);
 
 /* Exclusive scan of m uint32 counts into offs (device memory); tmp:
  * scan_tmp_bytes(m) bytes. */

@@ -190,6 +190,16 @@ void plb::host_populate(void *p, size_t bytes)
         if (t.joinable()) t.join();
 }
 
+void plb::host_populate_rows(double *const (&row)[4], size_t n)
+{
+    for (int c = 0; c < 4;) { /* rows that lie one after the other at once */
+        int m = 1;
+        while (c + m < 4 && row[c] && row[c + m] == row[c] + m * n) m++;
+        host_populate(row[c], sizeof(double) * n * m);
+        c += m;
+    }
+}
+
 /* ---------------------------------------------------------------- scan */
 
 constexpr int kScanThreads = 1024;
@@ -1199,12 +1209,7 @@ int plb_get_macros(plb_sim *s, double *rho, double *ux, double *uy, double *uz)
     k_get_macro<<<nblk(s->n, 256), 256, 0, s->stream>>>(s->macro, s->perm, s->npad, s->n, d);
     double *dst[4] = {rho, ux, uy, uz};
     cudaError_t e = cudaGetLastError();
-    for (int c = 0; c < 4;) { /* rows that lie one after the other at once */
-        int m = 1;
-        while (c + m < 4 && dst[c] && dst[c + m] == dst[c] + (size_t)m * s->n) m++;
-        host_populate(dst[c], sizeof(double) * (size_t)s->n * m);
-        c += m;
-    }
+    host_populate_rows(dst, (size_t)s->n);
     for (int c = 0; c < 4 && e == cudaSuccess; c++)
         if (dst[c])
             e = cudaMemcpyAsync(dst[c], d + (size_t)c * s->n, sizeof(double) * (size_t)s->n,
