@@ -36,12 +36,11 @@ BYTES_PER_NODE = {"fp64_exact": 376, "fp64": 376, "fp64_fma": 376, "fp32": 224,
                   "fp16dev": 148, "bf16dev": 148}
 
 
-def bytes_per_node(prec, num_node, order):
-    """The FP32 form keeps 16-bit words (36 bytes instead of 72) in row order
-    on domains that outgrow the L2."""
-    if prec == "fp32" and order == "reference" and num_node > 400000:
-        return 188
-    return BYTES_PER_NODE[prec]
+def bytes_per_node(prec, words):
+    """`words`: the handle's (Simulation.words).  Blocks with 16-bit neighbour
+    words read 36 bytes of words a node instead of 72."""
+    return round(BYTES_PER_NODE[prec] -
+                 36 * words["short_blocks"] / max(words["blocks"], 1), 1)
 
 
 # DRAM bytes (read + write) of one step-kernel launch come from one-pass ncu
@@ -316,6 +315,7 @@ def run_gpu(args, rank, world, local):
     kv = args.kernel_variant
     sim = P.Simulation(V, *dims, vs, tau=w["tau"], force=w["force"],
                        precision=prec, device=local, kernel_variant=kv)
+    words = sim.words()
     sim.init_dist_macro()
     stream = torch.cuda.ExternalStream(sim.stream, device=local)
     it = 0
@@ -410,9 +410,9 @@ def run_gpu(args, rank, world, local):
         device=local, kernel_variant=kv))
 
     peak, peak_kind = hbm_peak()
-    order = P.auto_ordering(N, dims[2], prec, local)
+    order = words["ordering"]
     traffic, traffic_src = recorded_traffic(args.workload, prec, N, order)
-    bpn = bytes_per_node(prec, N, order)
+    bpn = bytes_per_node(prec, words)
     achieved = bpn * N / (ms_step * 1e-3) / 1e9
     line = {
         "metric": METRIC, "value": round(value, 3), "unit": "MLUPS",
@@ -811,8 +811,7 @@ def run_precision(args):
         sim.sync()
         ms = e0.elapsed_time(e1)
         out[prec] = dict(mlups=round(sim.N * args.steps / (ms * 1e-3) / 1e6, 1),
-                         bytes_per_node=bytes_per_node(
-                             prec, sim.N, P.auto_ordering(sim.N, n, prec)),
+                         bytes_per_node=bytes_per_node(prec, sim.words()),
                          num_node=sim.N, device_bytes=sim.info()["device_bytes"])
         sim.close()
     flag, _, _ = P.sphere_pack_device(2, n, n, n, 8.0, 8.0, 0.20)

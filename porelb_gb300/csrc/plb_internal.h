@@ -201,7 +201,6 @@ struct StepArgs {
     void *fout;
     const uint32_t *nbr;  /* word_at() */
     const int2 *shorts;   /* by block of 256 nodes (see kWholeWords); may be NULL */
-    int rest;              /* the rest slot */
     const int *perm;      /* new -> reference index (density guard report) */
     long long npad;
     int n;
