@@ -811,10 +811,13 @@ k_batch_step(const BatchArgs a)
     const bool launch = Trig::waited(a.trigger);
     Trig::start(a.trigger);
     int2 base = make_int2(kWholeWords, 0);
-    if (W == kWordsShort) base = a.shorts[pb];
+    if (W == kWordsShort) base.x = a.shorts[pb].x;
     if (W == kWordsShort && base.x != kWholeWords) {
         uint32_t q[9];
-        if (valid) load_short(a.nbr, i, q);
+        if (valid) {
+            load_short(a.nbr, i, q);
+            base.y = a.shorts[pb].y; /* (with x in one load: 3% at 92k nodes) */
+        }
         pdl_wait(launch);
         if (valid) gather_short<T>((const T *)a.fin, q, a.npad, i, base, a.rest, raw);
     } else {
