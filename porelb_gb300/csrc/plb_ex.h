@@ -38,7 +38,7 @@
  * A node that is outside by its velocity alone is told apart: its moments
  * stand.
  *
- * Measured (256^3 pack, 5.87M nodes): 992 us a step (5.9 GLUPS) against 2204
+ * Measured (256^3 pack, 5.87M nodes): 990 us a step (5.9 GLUPS) against 2204
  * (2.66) with every add on the FP64 pipe and IEEE products made one by one
  * from FP64 bits; 24x20x16: 8.7 against 15 us.  Bound by the integer ALU and
  * FP64 pipes together, each about three quarters busy.

@@ -144,7 +144,7 @@ __device__ __forceinline__ void gather_words(const T *fin, long long np, long lo
     for (int j = 1; j < Q; j++) f[j] = fin[(long long)j * np + w[j - 1]];
 }
 
-/* the same two in one: the gathers go out as their words arrive */
+/* the same two in one: each gather waits for its own words alone */
 template <typename T>
 __device__ __forceinline__ void gather(const T *fin, const uint32_t *nbr,
                                        long long np, long long i, T (&f)[Q])
@@ -155,8 +155,8 @@ __device__ __forceinline__ void gather(const T *fin, const uint32_t *nbr,
 }
 
 /* The streamed values of node i (if valid), after the step before: WF loads
- * the neighbour words before the wait, else each gather goes out as its word
- * arrives after it (words_first_waves); `launch` triggers the next step's
+ * the neighbour words before the wait, else they are loaded after it and each
+ * gather waits for its own (words_first_waves); `launch` triggers the next step's
  * launch after the wait. */
 template <typename T, bool WF>
 __device__ __forceinline__ void stream_node(const void *fin, const uint32_t *nbr,
@@ -476,7 +476,7 @@ template <> struct StoreOf<PLB_BF16DEV> { using T = __nv_bfloat16; };
  * spill: FP16 at 92k nodes 2.94 against 2.75 us); the alternatives
  * unconstrained and 40.
  * Bit-exact FP64: 80 (its integer chains wait on themselves, so warps pay:
- * 5.8 GLUPS at 256^3 against 4.9 with 108 registers and 16 warps per SM; 64
+ * 5.9 GLUPS at 256^3 against 4.9 with 108 registers and 16 warps per SM; 64
  * registers spill: 5.7).  FMA FP64: unconstrained. */
 template <int PREC, int V, int W> struct MinBlocks {
     static constexpr bool dev = PREC == PLB_FP32 || PREC == PLB_FP16DEV || PREC == PLB_BF16DEV;
@@ -699,10 +699,9 @@ k_step(const StepArgs a)
     const bool launch = Trig::waited(a.trigger);
     Trig::start(a.trigger);
     if constexpr (PREC == PLB_FP64) {
-        /* one kernel for both: built apart, the form with the words after
-         * the wait spills 20 B at its 128 registers (348 against 341 us at
-         * 256^3); FP32 and 16-bit kernels are the ones with registers to
-         * lose to a branch */
+        /* one kernel for both, as fast as two (256^3 315.7 against 314.6 us,
+         * 24^3 2.68 against 2.83); FP32 and 16-bit kernels are the ones with
+         * registers to lose to a branch */
         if (a.words_first) stream_node<T, true>(a.fin, a.nbr, a.npad, i, i < a.n, launch, raw);
         else stream_node<T, false>(a.fin, a.nbr, a.npad, i, i < a.n, launch, raw);
     } else if constexpr (W == kWordsShort) {
@@ -1051,13 +1050,13 @@ void plan_step(int precision, int n, StepLaunch *l)
 }
 
 /* Threads per CTA of the plain step.  128 for the fixed-point and FMA FP64
- * forms; 256 for the others once 128-thread CTAs fill the device, since
- * warps of one CTA share instruction fetches (bit-exact form 1019 against
- * 1103 us at 256^3, FP16 at 22M nodes 575 against 648), and 128 below, where the finer grain
- * spreads better (bit-exact at 92k nodes 20.7 against 23.8 us, FP32 at 76k
- * 2.8 / 2.7, at 131k 3.8 / 4.2).  Domains that 64-thread CTAs cover with one
- * per SM take those: fewer warps share an SM's pipes (1.4k-9k nodes: FMA 7.0
- * against 7.7 us, FP64 2.8 / 3.1, bit-exact 9.4 / 9.8). */
+ * forms (FP64 at 256^3 319 us, with 256 threads 366); 256 for the others once
+ * 128-thread CTAs fill the device (bit-exact form 990 against 1101 us at
+ * 256^3, FP16 130 / 135), and 128 below, where the finer grain spreads better
+ * (at 92k nodes bit-exact 20.7 against 23.4 us, FP32 3.0 / 3.3).  Domains that
+ * 64-thread CTAs cover with one per SM take those: fewer warps share an SM's
+ * pipes (4.6k nodes: FMA 6.8 against 7.5 us, FP64 2.62 / 2.71, bit-exact 8.6 /
+ * 8.5). */
 template <int PREC>
 static int block_prec(int n)
 {
