@@ -235,8 +235,9 @@ struct Macro {
 };
 
 /* The collision from a node's moments (u shifted by the force): f(j) gives
- * the streamed values, store(j, x) takes the others. */
-template <bool NATIVE, typename Value, typename Store>
+ * the streamed values, store(j, x) takes the others.  Which products run on the
+ * FP64 pipe: EQ those of the equilibrium, RELAX those of the relaxation. */
+template <bool EQ, bool RELAX, typename Value, typename Store>
 __device__ __forceinline__ void relax_fp64_exact(const Coeffs &a, double rho, double u, double v,
                                                  double w, const Value &f, const Store &store)
 {
@@ -252,8 +253,8 @@ __device__ __forceinline__ void relax_fp64_exact(const Coeffs &a, double rho, do
 
     /* rest direction: e.u = 0 gives ((1 + 0) + 0) - 1.5 uv */
     {
-        const double feq = imul<NATIVE>(h0, dsub(1.0, uv15));
-        store(0, dadd(imul<NATIVE>(a.om1, f(0)), imul<NATIVE>(a0, feq)));
+        const double feq = imul<EQ>(h0, dsub(1.0, uv15));
+        store(0, dadd(imul<RELAX>(a.om1, f(0)), imul<RELAX>(a0, feq)));
     }
     /* pairs (J, J+1) with e_{J+1} = -e_J: 3 e.u, 4.5 e.u and (4.5 e.u) e.u
      * of the partner are exact negations / the same value. */
@@ -269,15 +270,15 @@ __device__ __forceinline__ void relax_fp64_exact(const Coeffs &a, double rho, do
                         : (J == 13) ? eu_ref<13>(u, v, w)
                         : (J == 15) ? eu_ref<15>(u, v, w)
                                     : eu_ref<17>(u, v, w);
-        const double t3 = imul<NATIVE>(3.0, eu);
-        const double c2 = imul<NATIVE>(imul<NATIVE>(4.5, eu), eu);
+        const double t3 = imul<EQ>(3.0, eu);
+        const double c2 = imul<EQ>(imul<EQ>(4.5, eu), eu);
         const double h = wclass(J) == 1 ? h1 : h2;
-        const double feqJ = imul<NATIVE>(h, dsub(dadd(dadd(1.0, t3), c2), uv15));
-        const double feqK = imul<NATIVE>(h, dsub(dadd(dsub(1.0, t3), c2), uv15));
+        const double feqJ = imul<EQ>(h, dsub(dadd(dadd(1.0, t3), c2), uv15));
+        const double feqK = imul<EQ>(h, dsub(dadd(dsub(1.0, t3), c2), uv15));
         const double AJ = ex(J) > 0 ? ap : (ex(J) < 0 ? am : a0);
         const double AK = ex(K) > 0 ? ap : (ex(K) < 0 ? am : a0);
-        store(J, dadd(imul<NATIVE>(a.om1, f(J)), imul<NATIVE>(AJ, feqJ)));
-        store(K, dadd(imul<NATIVE>(a.om1, f(K)), imul<NATIVE>(AK, feqK)));
+        store(J, dadd(imul<RELAX>(a.om1, f(J)), imul<RELAX>(AJ, feqJ)));
+        store(K, dadd(imul<RELAX>(a.om1, f(K)), imul<RELAX>(AK, feqK)));
     }
 }
 
@@ -305,8 +306,8 @@ __device__ __forceinline__ Macro collide_fp64_exact(double (&f)[Q],
     m.u = __ddiv_rn(ru, rho);
     m.v = __ddiv_rn(rv, rho);
     m.w = __ddiv_rn(rw, rho);
-    relax_fp64_exact<NATIVE>(a, rho, m.u, m.v, m.w, [&](int j) { return f[j]; },
-                             [&](int j, double x) { f[j] = x; });
+    relax_fp64_exact<NATIVE, NATIVE>(a, rho, m.u, m.v, m.w, [&](int j) { return f[j]; },
+                                     [&](int j, double x) { f[j] = x; });
     return m;
 }
 
@@ -493,9 +494,11 @@ template <int PREC, int V, int W> struct MinBlocks {
 
 /* The bit-exact collision of node i that left plb_ex.h's domain by its
  * velocity, from its moments: its streamed values, gathered again, are needed
- * one by one, and all 19 are stored again (128^3 with every node past the
- * range: 500 us a step, from the values alone 635).  Out of line, so the common
- * path keeps its registers. */
+ * one by one, and all 19 are stored again (128^3 with half or all of the nodes
+ * past the range: 449 and 480 us a step; from the values alone 662 and 635;
+ * with the equilibrium's products on the integer pipes too 522 and 503, with
+ * none there 440 and 531).  Out of line, so the common path keeps its
+ * registers. */
 __device__ __noinline__ void exact_node_fast(const double *fin, double *fout, const uint32_t *nbr,
                                              long long np, long long i, const Coeffs *run,
                                              double rho, double u, double v, double w)
@@ -504,8 +507,8 @@ __device__ __noinline__ void exact_node_fast(const double *fin, double *fout, co
     load_words<double>(nbr, np, i, at);
     auto value = [&](int j) { return fin[j == 0 ? i : (long long)j * np + at[j - 1]]; };
     auto store = [&](int j, double x) { __stcs(fout + (long long)j * np + i, x); };
-    if (run->exact_native) relax_fp64_exact<true>(*run, rho, u, v, w, value, store);
-    else relax_fp64_exact<false>(*run, rho, u, v, w, value, store);
+    if (run->exact_native) relax_fp64_exact<true, true>(*run, rho, u, v, w, value, store);
+    else relax_fp64_exact<true, false>(*run, rho, u, v, w, value, store);
 }
 
 /* The bit-exact collision of node i outside plb_ex.h's common domain, from
